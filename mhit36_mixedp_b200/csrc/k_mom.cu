@@ -369,12 +369,18 @@ __global__ void __launch_bounds__(MNT, 3) k_mom_batch(const __grid_constant__ Ba
   }
 }
 
-int mom_zchunk(const Geo& g, int requested) {
-  // Default chunk: 64 planes where that still leaves eight waves of three blocks on each of the
-  // 148 SMs (2.896 against 2.928 ms at 512^3), otherwise MZC.  Results do not depend on it.
+int mom_zchunk(const Geo& g, int requested, bool many) {
   if (requested > 0) return requested;
   const long long cols = (long long)((g.nx + MTX - 1) / MTX) * ((g.ny + MTY - 1) / MTY);
-  return cols * ((g.nz + 63) / 64) >= 8 * 148 * 3 ? 64 : MZC;
+  // 64 planes where that leaves eight waves of three blocks on each of the 148 SMs (2.896 against
+  // 2.928 ms at 512^3), MZC for one of many boxes that share the chip.
+  if (cols * ((g.nz + 63) / 64) >= 8 * 148 * 3) return 64;
+  if (many) return MZC;
+  // Smaller grids: the fewest planes in sequence, as k_phase, with three blocks per SM and four
+  // planes' time to fill the rings.  Measured, chunk of 32 -> the rule's: 64^3 33 -> 14 us (4
+  // planes), 128^3 55 -> 51 us (22), 192x64x128 60 -> 48 us (16), 256^3 unchanged (52 planes).
+  // Results do not depend on the chunk.
+  return best_zchunk(g.nz, cols, 3 * 148, 4);
 }
 
 dim3 mom_grid(const Geo& g, int zc) {
@@ -405,7 +411,7 @@ static cudaError_t launch_mom_t(const MomArgs& a, cudaStream_t st) {
     attr_set[dev] = 1;
   }
   MomArgs b = a;
-  b.zchunk = mom_zchunk(a.g, a.zchunk);
+  b.zchunk = mom_zchunk(a.g, a.zchunk, a.many);
   k_mom<PHI><<<mom_grid(a.g, b.zchunk), MNT, smem, st>>>(b);
   return cudaGetLastError();
 }

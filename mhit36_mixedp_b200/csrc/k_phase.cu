@@ -274,15 +274,20 @@ __global__ void __launch_bounds__(PNT, PMINB) k_phase_batch(const __grid_constan
   }
 }
 
-int phase_zchunk(const Geo& g, int requested) {
-  // Default chunk: 256 planes where that still leaves six waves of one block on each of the 148
-  // SMs (the four planes of warm-up below a chunk cost 1.6%: 2.27 against 2.31 ms at 512^3 with
-  // 128 planes), else 128 planes where that leaves eight waves (3% instead of 6%: 2.667 against
-  // 2.723 ms at 512^3 with 64), otherwise PZC.  Results do not depend on the chunk.
+int phase_zchunk(const Geo& g, int requested, bool many) {
   if (requested > 0) return requested;
   const long long cols = (long long)((g.nx + PTX - 1) / PTX) * ((g.ny + PTY - 1) / PTY);
-  if (cols * ((g.nz + 255) / 256) >= 6 * 148) return 256;
-  return cols * ((g.nz + 127) / 128) >= 8 * 148 ? 128 : PZC;
+  if (many) {
+    // one of many boxes that share the chip: long chunks, whose four planes of warm-up cost least
+    if (cols * ((g.nz + 255) / 256) >= 6 * 148) return 256;
+    return cols * ((g.nz + 127) / 128) >= 8 * 148 ? 128 : PZC;
+  }
+  // The even chunk with the fewest planes in sequence on an SM: waves of one block on each of the
+  // 148 SMs times the chunk with its four planes of warm-up (the shorter list of chunks on a tie).
+  // Measured, chunk of 64 -> the rule's: 128^3 87 -> 50 us (32 planes), 192x64x128 83 -> 37 us
+  // (22 planes), 256^3 345 -> 321 us (256 planes); 512^3 takes 256 planes (2.27 ms; 2.31 with 128).
+  // Results do not depend on the chunk.
+  return best_zchunk(g.nz, cols, 148, 4);
 }
 
 dim3 phase_grid(const Geo& g, int zc) {
@@ -314,7 +319,7 @@ cudaError_t launch_phase(const PhaseArgs& a, cudaStream_t st) {
   PhaseArgs b = a;
   b.dta = a.g.dt * a.alpha;
   b.dtb = a.g.dt * a.beta;
-  b.zchunk = phase_zchunk(a.g, a.zchunk);
+  b.zchunk = phase_zchunk(a.g, a.zchunk, a.many);
   const int zc = b.zchunk;
   if (zc % 2 || a.g.nz % 2) return cudaErrorInvalidValue;  // the plane loop runs two planes at a time
   kern<<<phase_grid(a.g, zc), PNT, smem, st>>>(b);

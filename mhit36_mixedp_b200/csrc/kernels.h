@@ -57,6 +57,25 @@ cudaError_t launch_combine(const float* p32, const float* d32, double* p64, size
 cudaError_t poisson_stage(const PoissonArgs& a, int stage, cudaStream_t st);
 bool poisson_size_supported(int n, bool is_x);
 
+// z planes per block of a stencil that marches `cols` columns of nz planes on `slots` resident
+// blocks and spends `warm` planes' time at the start of each chunk: the even chunk with the least
+// ceil(blocks / slots) (chunk + warm)
+inline int best_zchunk(int nz, long long cols, int slots, int warm) {
+  int best = nz + (nz & 1);
+  long long best_cost = -1;
+  for (int nch = 1; nch <= (nz + 1) / 2; ++nch) {
+    int zc = (nz + nch - 1) / nch;
+    zc += zc & 1;
+    const long long blocks = cols * ((nz + zc - 1) / zc);
+    const long long cost = (blocks + slots - 1) / slots * (zc + warm);
+    if (best_cost < 0 || cost < best_cost) {
+      best = zc;
+      best_cost = cost;
+    }
+  }
+  return best;
+}
+
 // ---------------------------------------------------------------- phase field
 struct PhaseArgs {
   Geo g;
@@ -68,6 +87,7 @@ struct PhaseArgs {
   double alpha, beta;
   int clamp;            // 1: phi clamped to [0,1] before the log
   int zchunk;           // z planes per block (0: default)
+  bool many = false;    // the box shares the chip with others (default chunk)
   double dta = 0, dtb = 0;  // dt alpha, dt beta (set by launch_phase)
 };
 cudaError_t launch_phase(const PhaseArgs& a, cudaStream_t st);
@@ -82,7 +102,7 @@ template <typename A> struct BatchArgs {
   int* counter;
   double alpha, beta;
 };
-int phase_zchunk(const Geo& g, int requested);  // the z chunk launch_phase uses
+int phase_zchunk(const Geo& g, int requested, bool many);  // the z chunk launch_phase uses
 dim3 phase_grid(const Geo& g, int zc);           // its tiles: x, y, z chunk
 cudaError_t launch_phase_batch(const BatchArgs<PhaseArgs>& b, bool clamp, int nsm, cudaStream_t st);
 
@@ -97,13 +117,14 @@ struct MomArgs {
   const DevScalars* sc;
   double alpha, beta;
   int zchunk;                // z planes per block (0: default)
+  bool many = false;         // the box shares the chip with others (default chunk)
   // TMA tensor maps of u, v, w and phi^{n+1} (mom_field_maps); when `tma` is set the blocks whose
   // rings need no periodic wrap in x and y fill them with TMA boxes instead of per-thread copies
   int tma = 0;
   CUtensorMap tmu, tmv, tmw, tmphi;
 };
 cudaError_t launch_mom(const MomArgs& a, cudaStream_t st);
-int mom_zchunk(const Geo& g, int requested);  // the z chunk launch_mom uses
+int mom_zchunk(const Geo& g, int requested, bool many);  // the z chunk launch_mom uses
 dim3 mom_grid(const Geo& g, int zc);           // its tiles: x, y, z chunk
 cudaError_t launch_mom_batch(const BatchArgs<MomArgs>& b, bool phi, int nsm, cudaStream_t st);
 // tensor map of an x-fastest nx*ny*nz float64 field with the ring box of k_mom (36 x 10 for the

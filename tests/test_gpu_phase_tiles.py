@@ -1,0 +1,42 @@
+"""Phase and momentum stages on boxes whose tiles and z chunks do not divide the grid.
+
+The stencils march tiles of x-y cells over chunks of z planes chosen from the grid size; these boxes
+leave a partial last tile in x or y, a short last chunk, or a chunk of two planes.  Each stage is one
+FP64 evaluation of the oracle's expressions, so the usual 1e-12 of the buffer's maximum applies.
+"""
+import numpy as np
+import pytest
+
+from mhit36_mixedp_b200 import Params, Solver, synth
+from oracle import mhit_oracle as orc
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-12
+
+
+def rel(a, b):
+    return float(np.max(np.abs(a - b)) / np.max(np.abs(b)))
+
+
+@pytest.mark.parametrize("clamp", [0, 1])
+@pytest.mark.parametrize("shape", [(16, 16, 16), (16, 64, 16), (64, 16, 128), (192, 64, 128), (32, 192, 64), (64, 128, 16)])
+def test_stencil_stages_on_ragged_boxes(gpu, shape, clamp):
+    nx, ny, nz = shape
+    dx = 2 * np.pi / nx
+    u, v, w = synth.solenoidal_velocity(nx, 3, ny=ny, nz=nz)
+    # one smooth interface that crosses every tile and chunk boundary, phi strictly inside (0, 1)
+    z, y, x = np.meshgrid(*(np.arange(n) * 2 * np.pi / n for n in (nz, ny, nx)), indexing="ij")
+    phi = 0.5 * (1 - np.tanh((np.cos(x) + np.cos(y) + np.cos(z)) / (2 * dx)))
+    prm = dict(nx=nx, ny=ny, nz=nz, dt=2e-4, mu=0.004, phiflag=1, sigma=0.3, acdi_clamp=clamp)
+    op = orc.Params(**prm)
+    st = orc.new_state(op, u, v, w, phi=phi)
+    with Solver(Params(**prm)) as s:
+        s.upload(u, v, w, phi)
+        orc.phase_step(op, st)
+        s.run_stage("phase")
+        assert rel(s.buffer("phin"), st.phi) < TOL
+        assert rel(s.buffer("rphi"), st.rhsphi_o) < TOL
+        orc.momentum_step(op, st, orc.forcing_tables(op))
+        s.run_stage("momentum")
+        for f, name in (("un", "u"), ("vn", "v"), ("wn", "w")):
+            assert rel(s.buffer(f), getattr(st, name)) < TOL
