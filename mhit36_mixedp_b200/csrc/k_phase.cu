@@ -1,21 +1,19 @@
 // ACDI phase-field transport: multi/main.f90:522-636 in one kernel.
 //
 // The reference makes five passes with three stored intermediates (psidi, tanh_psi and the
-// three normal components) and six halo exchanges.  Here a block owns a TX x TY column of
-// cells and marches up a chunk of z planes.  It has one thread per position of the tile plus
-// its x/y halo of 2 ((TX+4)(TY+4) threads), and each thread keeps its own z column in
-// registers:
+// three normal components) and six halo exchanges.  Here a block owns a PTX x PTY column of
+// cells and marches up a chunk of z planes.  It has one thread per vertical pair of positions of
+// the tile plus its x/y halo of 2, and each thread keeps its two z columns in registers:
 //   phi  planes k-1..k+3 (k+3 loaded one plane ahead)
 //   psi  = eps log((min(phi,1)+1e-16)/(1-min(phi,1)+1e-16))            (:527-528), k..k+2
 //   Fz   of F = 1/4 (1 - t^2) n/(|n|+1e-16), n = central psi differences (:559-561,
 //        :586-589, :609-614), t = tanh(psi/(2 eps)) (:530),               planes k-1..k+1
-//        (n/(|n|+1e-16) is evaluated as n rsqrt(|n|^2), see F_of)
 // Only x/y neighbours go through shared memory: psi(k+1), phi(k) and Fx, Fy(k), each
-// double-buffered.  Every shared read of plane k's iteration reads what the previous
-// iteration wrote, so one barrier per plane suffices.  psi is evaluated on the halo of 2 and F
-// on the halo of 1 (factors (TX+4)(TY+4)/(TX TY) and (TX+2)(TY+2)/(TX TY)); threads are
-// numbered so that the TX x TY output cells fill whole warps, then the F ring, then the outer
-// psi-only ring.  The kernel writes only phi^{n+1} and rhsphi_o.
+// double-buffered, and the output cells' u, v, w and rhsphi_o, copied there with cp.async one
+// plane ahead.  Every shared read of plane k's iteration reads what the previous iteration wrote
+// or fetched, so one barrier per plane suffices.  psi is evaluated on the halo of 2 and F on the
+// halo of 1; threads are numbered so that the output pairs fill whole warps, then the F ring,
+// then the outer psi-only ring.  The kernel writes only phi^{n+1} and rhsphi_o.
 //
 // t is evaluated in closed form: tanh(log(r)/2) = (r-1)/(r+1) with r = (val+1e-16)/(1-val+1e-16)
 // gives t = (2 val - 1)/(1 + 2e-16) exactly in real arithmetic; in float64 it agrees with the
@@ -27,6 +25,8 @@
 //
 // gamma = 1.0*gumax is read from the device scalars written by the previous projection
 // (:536, :998-1002); u, v, w are the stored fields minus the lazily removed mean.
+#include <cuda_pipeline.h>
+
 #include <type_traits>
 
 #include "common.cuh"
@@ -34,30 +34,80 @@
 
 namespace mhit {
 
-// 32 x 16 output cells per block, one block per SM (two blocks of 16 x 16 or 16 x 12 outputs,
-// with more halo, were slower: 2.90 and 3.08 against 2.64 ms at 512^3)
-constexpr int PTX = 32, PTY = 16;  // output cells per block in x, y
+// 32 x 24 output cells per block, one block per SM, two vertically adjacent cells per thread.  The
+// kernel is bound by the latency of its FP64 chains (reciprocal, logarithm polynomial, reciprocal
+// square root) and of its loads at the 16 to 24 warps an SM holds.  One cell per thread and loads
+// in the iteration that uses them (32 x 16 tiles, 23 warps) issued 62% of the cycles and took
+// 2.34 ms at 512^3 and 331 us at 256^3.  Now each thread carries two independent chains, psi is
+// evaluated on 1.31 instead of 1.41 and F on 1.15 instead of 1.20 cells per output cell, the y
+// neighbours inside a pair come from registers, one barrier serves half again as many cells, and
+// the fields of the next plane are fetched a whole plane ahead: 1.97 ms and 264 us (without the
+// fetch 2.18 ms and 288 us).  ncu at 256^3: 12.3 -> 8.3 warp instructions per cell, FP64 pipe 43%,
+// issue 54%.  504 threads leave 128 registers: 32 x 32 tiles (648 threads, 80 registers) spill and
+// take 2.01 ms, two 32 x 12 blocks per SM 2.29 ms (without the fetch).
+constexpr int PTX = 32, PTY = 24;  // output cells per block in x, y
 constexpr int PMINB = 1;           // resident blocks per SM
 constexpr int PHX = PTX + 4, PHY = PTY + 4;  // positions with the halo of 2
-constexpr int PNT = PHX * PHY;               // threads per block = positions
-constexpr int PNI = PTX * PTY;               // output cells
-constexpr int PNF = (PHX - 2) * (PHY - 2);   // F positions (halo 1)
+constexpr int PPOS = PHX * PHY;              // positions of a shared plane
+constexpr int PNT = PHX * PHY / 2;           // threads per block: one per pair of rows
+constexpr int PNO = PTX * PTY / 2;           // threads with two output cells
+constexpr int PNF = PNO + 2 * PTX + 4 + 2 * (PTY / 2);  // ... plus those that evaluate F on the halo of 1
+constexpr int PUNROLL = 2;  // two-plane bodies per loop iteration (1: 2.07 ms at 512^3)
+// one plane of the output cells' u (one column more), v (one row more), w(k+1) and rhs_o in shared
+// memory, fetched with cp.async one plane ahead
+constexpr int PUX = PTX + 2;
+constexpr int PSU = 0, PSV = PSU + PTY * PUX, PSW = PSV + (PTY + 1) * PTX, PSR = PSW + PTY * PTX,
+              PSTG = PSR + PTY * PTX;
+constexpr size_t PSMEM = sizeof(double) * (8 * PPOS + 2 * PSTG);  // psi, phi, Fx, Fy and the staged fields, twice each
 constexpr int PZC = 64;                      // default z planes per block
 constexpr double ENUM = 1.0e-16;
 constexpr double TNORM = 1.0 / (1.0 + 2.0 * ENUM);
 
-// a / b for b in [1e-16, 2] to within an ulp, in FMAs: the reciprocal from an FP32 seed (24
-// bits) refined by two Newton-Raphson steps r <- r + r (1 - b r) (48, then 53 bits), the quotient
-// q = a r corrected once with its residual, q <- q + r (a - b q) (Markstein's scheme).  Used for
-// psi's quotient, whose error enters the normals only through psi differences.
-__device__ __forceinline__ double div_nr(double a, double b) {
-  double r = (double)__fdividef(1.0f, (float)b);
-  double e = __fma_rn(-b, r, 1.0);
-  r = __fma_rn(r, e, r);
-  e = __fma_rn(-b, r, 1.0);
-  r = __fma_rn(r, e, r);
-  const double q = a * r;
-  return __fma_rn(r, __fma_rn(-b, q, a), q);
+// log(a/b) for finite b > 0 and a > 0 (a = 0: -inf, a < 0 or NaN: NaN), to an ulp or two, without
+// branches, conversions or a separate quotient: with k the integer nearest to the difference of
+// the operands' piecewise-linear log2 (exponent and mantissa fields of the high words) and
+// a' = a 2^-k, a'/b lies in [0.66, 1.51] and
+//   log(a/b) = k log 2 + 2 atanh(s),  s = (a' - b)/(a' + b), |s| < 0.201,
+// a' - b exact (Sterbenz).  2 atanh(s) = 2 s (1 + z Q(z)), z = s^2, Q the degree-7 interpolant of
+// the series 1/3 + z/5 + z^2/7 + ... at the Chebyshev nodes of [0, 0.0415] (2^-60 of the sum).
+// The quotient is one Newton-Raphson step on the approximate reciprocal and one residual
+// correction.
+template <bool POSITIVE> __device__ __forceinline__ double log_ratio(double a, double b) {
+  const int ha = __double2hiint(a), hb = __double2hiint(b);
+  const int k = (int)((unsigned)ha - (unsigned)hb + (1u << 19)) >> 20;
+  const double as = __hiloint2double((int)((unsigned)ha - ((unsigned)k << 20)), __double2loint(a));
+  const double kd = __hiloint2double(0x43380000, k ^ 0x80000000) - 6755401588539392.0;  // k as a double
+  const double n = as - b, d = as + b;
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+  r = __fma_rn(__fma_rn(-d, r, 1.0), r, r);
+  double s = n * r;
+  s = __fma_rn(__fma_rn(-d, s, n), r, s);
+  const double z = s * s;
+  double q = 0.06839733963975679;
+  q = __fma_rn(q, z, 0.06600187405442207);
+  q = __fma_rn(q, z, 0.07694675390670448);
+  q = __fma_rn(q, z, 0.09090862660038017);
+  q = __fma_rn(q, z, 0.11111111603983777);
+  q = __fma_rn(q, z, 0.14285714283150056);
+  q = __fma_rn(q, z, 0.20000000000005075);
+  q = __fma_rn(q, z, 0.3333333333333333);
+  const double t = s + s;
+  // log 2 in two parts, the first exact in its products with k
+  const double hi = __fma_rn(kd, 0.6931471805598903, t);
+  const double carry = __fma_rn(kd, 0.6931471805598903, -hi) + t;
+  const double lo = __fma_rn(kd, 5.497923018708371e-14, __fma_rn(t * z, q, carry));
+  const double l = hi + lo;
+  if (POSITIVE) return l;
+  return a > 0.0 ? l : (a == 0.0 ? -INFINITY : NAN);
+}
+
+// 1/sqrt(x) for normal x > 0: the approximate reciprocal square root and one third-order step
+__device__ __forceinline__ double rsqrt_fast(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = __fma_rn(-(x * y), y, 1.0);
+  return __fma_rn(y * e, __fma_rn(0.375, e, 0.5), y);
 }
 
 __device__ __forceinline__ int pmodi(int x, int n) {
@@ -65,41 +115,39 @@ __device__ __forceinline__ int pmodi(int x, int n) {
   return x < 0 ? x + n : x;
 }
 
-// position of ring element r of the w x h rectangle perimeter starting at (x0, y0): top row,
-// bottom row, left column, right column
-__device__ __forceinline__ void ring_pos(int r, int x0, int y0, int w, int h, int& x, int& y) {
-  if (r < w) { x = x0 + r; y = y0; return; }
-  r -= w;
-  if (r < w) { x = x0 + r; y = y0 + h - 1; return; }
-  r -= w;
-  if (r < h - 2) { x = x0; y = y0 + 1 + r; return; }
-  r -= h - 2;
-  x = x0 + w - 1;
-  y = y0 + 1 + r;
-}
-
 // One z column of PTX x PTY cells, tile (bx, by), chunk bz, of the box a; dta, dtb = dt alpha,
 // dt beta of the AB2 update.
 template <bool CLAMP>
 __device__ __forceinline__ void phase_tile(const PhaseArgs& a, double dta, double dtb, int bx, int by, int bz,
                                            unsigned char* smraw) {
-  // thread -> position (hx, hy) in the (PHX x PHY) grid of the tile with its halo
+  // thread -> column hx and row pair (rows 2 r, 2 r + 1) of the (PHX x PHY) grid of the tile with
+  // its halo: first the output pairs (whole warps), then the pairs that add F on the halo of 1
+  // (bottom and top row pair, of which only the inner row does; columns 1 and PTX + 2), then the
+  // psi-only columns 0 and PTX + 3
   const int tid = threadIdx.x;
-  int hx, hy;
-  if (tid < PNI) {
+  int hx, r;
+  if (tid < PNO) {
     hx = 2 + tid % PTX;
-    hy = 2 + tid / PTX;
+    r = 1 + tid / PTX;
+  } else if (tid < PNO + 2 * (PTX + 2)) {
+    const int e = tid - PNO;
+    hx = 1 + e % (PTX + 2);
+    r = e < PTX + 2 ? 0 : PHY / 2 - 1;
   } else if (tid < PNF) {
-    ring_pos(tid - PNI, 1, 1, PHX - 2, PHY - 2, hx, hy);
+    const int e = tid - PNO - 2 * (PTX + 2);
+    hx = e < PTY / 2 ? 1 : PTX + 2;
+    r = 1 + e % (PTY / 2);
   } else {
-    ring_pos(tid - PNF, 0, 0, PHX, PHY, hx, hy);
+    const int e = tid - PNF;
+    hx = e < PHY / 2 ? 0 : PTX + 3;
+    r = e % (PHY / 2);
   }
-  const int q = hy * PHX + hx;  // this position in a shared plane
+  const int q = 2 * r * PHX + hx;  // lower cell's position in a shared plane; the upper one's is q + PHX
   // shared planes at this position: psi[2], phi[2], Fx[2], Fy[2]
   double* sps = reinterpret_cast<double*>(smraw) + q;
-  double* sph = sps + 2 * PNT;
-  double* sfx = sph + 2 * PNT;
-  double* sfy = sfx + 2 * PNT;
+  double* sph = sps + 2 * PPOS;
+  double* sfx = sph + 2 * PPOS;
+  double* sfy = sfx + 2 * PPOS;
 
   const Geo& g = a.g;
   const int nx = g.nx, ny = g.ny, nz = g.nz;
@@ -107,11 +155,12 @@ __device__ __forceinline__ void phase_tile(const PhaseArgs& a, double dta, doubl
   const int i0 = bx * PTX, j0 = by * PTY;
   const int zc = a.zchunk > 0 ? a.zchunk : PZC;
   const int k0 = bz * zc, k1 = min(k0 + zc, nz);
-  const int i = i0 - 2 + hx, j = j0 - 2 + hy;
-  const int col = pmodi(j, ny) * nx + pmodi(i, nx);
+  const int i = i0 - 2 + hx, j = j0 - 2 + 2 * r;  // lower cell; j and ny are even
+  const int ic = pmodi(i, nx), jc = pmodi(j, ny);
+  const int col = jc * nx + ic;                   // the upper cell's column is col + nx
   const bool frole = tid < PNF;
-  const bool orole = tid < PNI && i < nx && j < ny;
-  const double eps = g.eps;
+  const bool fa = frole && r >= 1, fb = frole && r < PHY / 2 - 1;
+  const bool orole = tid < PNO && i < nx && j < ny;
   const double* __restrict__ phig = a.phi;
 
   auto clampv = [](double ph) {
@@ -119,34 +168,26 @@ __device__ __forceinline__ void phase_tile(const PhaseArgs& a, double dta, doubl
     if (CLAMP) val = fmax(val, 0.0);
     return val;
   };
-  auto psi_of = [&](double ph) {  // multi/main.f90:527-528
+  // psi / eps of multi/main.f90:527-528 (only the direction of its gradient is used)
+  auto psi_of = [&](double ph) {
     const double val = clampv(ph);
-    return eps * log(div_nr(val + ENUM, 1.0 - val + ENUM));
+    return log_ratio<CLAMP>(val + ENUM, 1.0 - val + ENUM);
   };
-  // F of this position at one plane (multi/main.f90:530, 559-561, 586-589, 609-614): Q the
-  // plane's shared psi at this position, dz the psi difference along z, ph/ps this position's
-  // phi/psi.  The fused multiply-adds are written out, so the rounding does not depend on how
-  // the compiler contracts each copy of the loop body.
-  auto F_of = [&](const double* __restrict__ Q, double dz, double ph, double ps, double& fx, double& fy,
-                  double& fz) {
-    double nxr = Q[1] - Q[-1];
-    double nyr = Q[PHX] - Q[-PHX];
-    double nzr = dz;
-    const double n2 = __fma_rn(nzr, nzr, __fma_rn(nyr, nyr, __dmul_rn(nxr, nxr)));
-    // n/(|n| + 1e-16) as n rsqrt(|n|^2), 0 for n = 0: one reciprocal square root instead of a
-    // square root and a division (k_phase 2.58 -> 2.38 ms at 512^3).  It differs from the
-    // reference's quotient by 1e-16/|n| relative: far below rounding where the interface makes
-    // |n| large, and where psi is flat (|n| tiny) 1/4 (1 - t^2) ~ phi (1 - phi) ~ 0 multiplies it.
-    const double normag = n2 > 0.0 ? rsqrt(n2) : 0.0;
-    nxr = nxr * normag;
-    nyr = nyr * normag;
-    nzr = nzr * normag;
+  // F of one cell at one plane (multi/main.f90:530, 559-561, 586-589, 609-614) from the psi
+  // differences dx, dy, dz and its phi, psi.  n/(|n| + 1e-16) is n rsqrt(|n|^2), 0 for n = 0: it
+  // differs from the reference's quotient by 1e-16/|n| relative, far below rounding where the
+  // interface makes |n| large, and where psi is flat (|n| tiny) 1/4 (1 - t^2) ~ phi (1 - phi) ~ 0
+  // multiplies it.  The fused multiply-adds are written out, so the rounding does not depend on
+  // how the compiler contracts each copy of the loop body.
+  auto F_of = [&](double dx, double dy, double dz, double ph, double ps, double& fx, double& fy, double& fz) {
+    const double n2 = __fma_rn(dz, dz, __fma_rn(dy, dy, __dmul_rn(dx, dx)));
+    const double normag = (n2 > 0.0 && n2 <= 1.7976931348623157e308) ? rsqrt_fast(n2) : 0.0;
     const double val = clampv(ph);
-    const double tt = (ps == ps) ? (2.0 * val - 1.0) * TNORM : ps;
-    const double fac = 0.25 * __fma_rn(-tt, tt, 1.0);
-    fx = fac * nxr;
-    fy = fac * nyr;
-    fz = fac * nzr;
+    const double tt = (ps == ps) ? __fma_rn(2.0, val, -1.0) * TNORM : ps;
+    const double fac = __dmul_rn(__dmul_rn(0.25, __fma_rn(-tt, tt, 1.0)), normag);
+    fx = __dmul_rn(dx, fac);
+    fy = __dmul_rn(dy, fac);
+    fz = __dmul_rn(dz, fac);
   };
 
   const double gamma = 1.0 * a.sc->gumax;
@@ -154,94 +195,130 @@ __device__ __forceinline__ void phase_tile(const PhaseArgs& a, double dta, doubl
   const double dxi = g.dxi, ddxi = g.ddxi;
   const double hdxi = 0.5 * dxi;  // (x*0.5)*dxi == x*(0.5*dxi) exactly
   // the right-hand side's constant factors, applied once per sum of terms (see the output block)
-  const double c_lap = gamma * (eps * ddxi), c_shp = gamma * -hdxi;
-  int c = k0 * plane + col;  // own cell (output role)
+  const double c_lap = gamma * (g.eps * ddxi), c_shp = gamma * -hdxi;
+  int c = k0 * plane + col;  // lower cell (output role)
   const int dux = (i + 1 == nx) ? 1 - nx : 1;
-  const int dvy = (j + 1 == ny) ? (1 - ny) * nx : nx;
-  double w0 = orole ? __ldg(a.w + c) : 0.0;
+  const int dvy = (j + 2 == ny) ? (2 - ny) * nx : 2 * nx;  // the row above the pair
+  // staged fields of this pair; the pairs at the tile's or the box's upper edges also fetch the
+  // column (row) beyond it
+  const int lx = hx - 2, ly = 2 * (r - 1);
+  double* const stg = reinterpret_cast<double*>(smraw) + 8 * PPOS;
+  const bool uedge = lx == PTX - 1 || i + 1 == nx, vedge = ly + 2 == PTY || j + 2 == ny;
+  const int su = PSU + ly * PUX + lx, sv = PSV + ly * PTX + lx, sw = PSW + ly * PTX + lx, sr = PSR + ly * PTX + lx;
+  auto stage = [&](double* d, int k, int cc) {  // plane k, whose lower cell is cc, into the slot at d
+    const int cw = (k + 1 == nz) ? cc - (nz - 1) * plane : cc + plane;
+    __pipeline_memcpy_async(d + su, a.u + cc, 8);
+    __pipeline_memcpy_async(d + su + PUX, a.u + cc + nx, 8);
+    if (uedge) {
+      __pipeline_memcpy_async(d + su + 1, a.u + cc + dux, 8);
+      __pipeline_memcpy_async(d + su + PUX + 1, a.u + cc + nx + dux, 8);
+    }
+    __pipeline_memcpy_async(d + sv, a.v + cc, 8);
+    __pipeline_memcpy_async(d + sv + PTX, a.v + cc + nx, 8);
+    if (vedge) __pipeline_memcpy_async(d + sv + 2 * PTX, a.v + cc + dvy, 8);
+    __pipeline_memcpy_async(d + sw, a.w + cw, 8);
+    __pipeline_memcpy_async(d + sw + PTX, a.w + cw + nx, 8);
+    __pipeline_memcpy_async(d + sr, a.rphio + cc, 8);
+    __pipeline_memcpy_async(d + sr + PTX, a.rphio + cc + nx, 8);
+  };
+  double wa0 = orole ? __ldg(a.w + c) : 0.0, wb0 = orole ? __ldg(a.w + c + nx) : 0.0;
+
+  // Right-hand side and update of one output cell: p its phi and its six neighbours', the face
+  // velocities, and the sum of the F differences.  multi/main.f90:551-557 and :609-614 with each
+  // group's constant factor taken out of its sum (the same expression up to rounding: a few ulp
+  // of the terms, far inside the 1e-12 parity bound):
+  //   rhs = -dxi/2 sum_d (u_d+ (phi+ + phi) - u_d (phi + phi-))                 advection
+  //         + gamma eps ddxi (sum of the six neighbours - 6 phi)                diffusion
+  //         - gamma dxi/2 sum_d (F_d+ - F_d-)                                   sharpening
+  auto out_cell = [&](int cc, double p0, double pxp, double pxm, double pyp, double pym, double pzp, double pzm,
+                      double u_0, double u_x, double v_0, double v_y, double w_0, double w_z, double shp, double ro) {
+    const double adv = (__fma_rn(u_x, pxp + p0, -u_0 * (p0 + pxm)) + __fma_rn(v_y, pyp + p0, -v_0 * (p0 + pym))) +
+                       __fma_rn(w_z, pzp + p0, -w_0 * (p0 + pzm));
+    const double lap = ((pxp + pxm) + (pyp + pym)) + __fma_rn(-6.0, p0, pzp + pzm);
+    const double rhs = __fma_rn(-hdxi, adv, __fma_rn(c_lap, lap, c_shp * shp));
+    // :625-626
+    a.phin[cc] = __fma_rn(dta, rhs, __fma_rn(-dtb, ro, p0));
+    a.rphio[cc] = rhs;
+  };
 
   // Iteration k computes psi(k+2), F(k+1) and the output plane k.  The loop starts four planes
   // below the chunk: k0-4 and k0-3 only fill psi(k0-2), psi(k0-1), k0-2 and k0-1 add F(k0-1),
   // F(k0).  Every psi and F is thus evaluated by the loop body, so the values of a plane do
-  // not depend on where a z chunk starts.  Register state entering iteration k: phi k-1..k+2,
-  // psi k, k+1, Fz k-1, k.
-  double f_m1 = 0.0, f_0 = 0.0, f_p1 = 0.0, f_p2 = phig[pmodi(k0 - 2, nz) * plane + col];
-  double s_0 = 0.0, s_p1 = 0.0, z_m1 = 0.0, z_0 = 0.0;
-  int o3 = pmodi(k0 - 1, nz) * plane + col;  // phi(k+3) of the first iteration
+  // not depend on where a z chunk starts.  Register state of each cell entering iteration k: phi
+  // k-1..k+2, psi k, k+1, Fz k-1, k and Fy k.
+  int o3 = pmodi(k0 - 2, nz) * plane + col;
+  double fam1 = 0.0, fa0 = 0.0, fap1 = 0.0, fap2 = phig[o3];
+  double fbm1 = 0.0, fb0 = 0.0, fbp1 = 0.0, fbp2 = phig[o3 + nx];
+  double sa0 = 0.0, sap1 = 0.0, zam1 = 0.0, za0 = 0.0, ya0 = 0.0;
+  double sb0 = 0.0, sbp1 = 0.0, zbm1 = 0.0, zb0 = 0.0, yb0 = 0.0;
+  o3 = pmodi(k0 - 1, nz) * plane + col;  // phi(k+3) of the first iteration
 
   // One plane of the loop; P is the parity of k, so the double-buffer slots are compile-time
-  // offsets: slot(k) = slot(k + 2) = P PNT, slot(k + 1) = (1 - P) PNT.
+  // offsets: slot(k) = slot(k + 2) = P PPOS, slot(k + 1) = (1 - P) PPOS.
   auto plane_iter = [&](auto par, int k) {
     constexpr int P = decltype(par)::value;
-    constexpr int SK = P * PNT, SK1 = (1 - P) * PNT;
+    constexpr int SK = P * PPOS, SK1 = (1 - P) * PPOS;
     const bool out = orole && k >= k0;
-    const double f_p3 = (k + 1 < k1) ? phig[o3] : 0.0;
+    double fap3 = 0.0, fbp3 = 0.0;
+    if (k + 1 < k1) {
+      fap3 = phig[o3];
+      fbp3 = phig[o3 + nx];
+    }
     o3 += plane;
     if (o3 >= ntot) o3 -= ntot;
-    double u0 = 0, uxp = 0, v0 = 0, vyp = 0, wzp = 0, ro = 0;
-    if (out) {
-      const int cz = (k + 1 == nz) ? c - (nz - 1) * plane : c + plane;
-      u0 = __ldg(a.u + c);
-      uxp = __ldg(a.u + c + dux);
-      v0 = __ldg(a.v + c);
-      vyp = __ldg(a.v + c + dvy);
-      wzp = __ldg(a.w + cz);
-      ro = a.rphio[c];
-    }
-    // psi(k+2) of this position; phi(k+1) for the next plane's neighbours
-    const double s_p2 = psi_of(f_p2);
-    sps[SK] = s_p2;
-    sph[SK1] = f_p1;
+    // plane k+1's fields go out now; they land before the barrier that ends this iteration
+    if (orole && k + 1 >= k0 && k + 1 < k1) stage(stg + (1 - P) * PSTG, k + 1, k >= k0 ? c + plane : c);
+    __pipeline_commit();
+    // psi(k+2) of both cells; phi(k+1) for the next plane's neighbours
+    const double sap2 = psi_of(fap2), sbp2 = psi_of(fbp2);
+    sps[SK] = sap2;
+    sps[SK + PHX] = sbp2;
+    sph[SK1] = fap1;
+    sph[SK1 + PHX] = fbp1;
     // F(k+1) from the shared psi(k+1) (written last iteration) and the own psi(k+2) - psi(k)
-    double z_p1 = 0.0;
-    if (frole && k >= k0 - 2) {
-      double fx, fy;
-      F_of(sps + SK1, s_p2 - s_0, f_p1, s_p1, fx, fy, z_p1);
-      sfx[SK1] = fx;
-      sfy[SK1] = fy;
+    double zap1 = 0.0, zbp1 = 0.0, yap1 = 0.0, ybp1 = 0.0;
+    if (k >= k0 - 2) {
+      const double* Q = sps + SK1;
+      double fx;
+      if (fa) {
+        F_of(Q[1] - Q[-1], sbp1 - Q[-PHX], sap2 - sa0, fap1, sap1, fx, yap1, zap1);
+        sfx[SK1] = fx;
+        sfy[SK1] = yap1;
+      }
+      if (fb) {
+        F_of(Q[PHX + 1] - Q[PHX - 1], Q[2 * PHX] - sap1, sbp2 - sb0, fbp1, sbp1, fx, ybp1, zbp1);
+        sfx[SK1 + PHX] = fx;
+        sfy[SK1 + PHX] = ybp1;
+      }
     }
-    // output plane k from the shared phi(k), Fx/Fy(k) and the own column
+    // output plane k from the shared phi(k), Fx/Fy(k) and the own columns
     if (out) {
-      const double u_0 = u0 - mu_, u_x = uxp - mu_, v_0 = v0 - mv_, v_y = vyp - mv_;
-      const double w_0 = w0 - mw_, w_z = wzp - mw_;
       const double* P0 = sph + SK;
-      const double p0 = f_0;
-      const double pxp = P0[1], pxm = P0[-1], pyp = P0[PHX], pym = P0[-PHX];
-      const double pzp = f_p1, pzm = f_m1;
-      // multi/main.f90:551-557 and :609-614, with each group's constant factor taken out of its
-      // sum (the same expression up to rounding: a few ulp of the terms, far inside the 1e-12
-      // parity bound):
-      //   rhs = -dxi/2 sum_d (u_d+ (phi+ + phi) - u_d (phi + phi-))                 advection
-      //         + gamma eps ddxi (sum of the six neighbours - 6 phi)                diffusion
-      //         - gamma dxi/2 sum_d (F_d+ - F_d-)                                   sharpening
       const double* Fx = sfx + SK;
       const double* Fy = sfy + SK;
-      const double adv = (__fma_rn(u_x, pxp + p0, -u_0 * (p0 + pxm)) + __fma_rn(v_y, pyp + p0, -v_0 * (p0 + pym))) +
-                         __fma_rn(w_z, pzp + p0, -w_0 * (p0 + pzm));
-      const double lap = ((pxp + pxm) + (pyp + pym)) + __fma_rn(-6.0, p0, pzp + pzm);
-      const double shp = ((Fx[1] - Fx[-1]) + (Fy[PHX] - Fy[-PHX])) + (z_p1 - z_m1);
-      const double rhs = __fma_rn(-hdxi, adv, __fma_rn(c_lap, lap, c_shp * shp));
-      // :625-626
-      a.phin[c] = __fma_rn(dta, rhs, __fma_rn(-dtb, ro, p0));
-      a.rphio[c] = rhs;
-      w0 = wzp;
+      const double* G = stg + P * PSTG;
+      const double va = G[sv], vc = G[sv + 2 * PTX], ua = G[su], uax = G[su + 1], ub = G[su + PUX], ubx = G[su + PUX + 1];
+      const double waz = G[sw], wbz = G[sw + PTX], roa = G[sr], rob = G[sr + PTX];
+      const double v_b = G[sv + PTX] - mv_;
+      out_cell(c, fa0, P0[1], P0[-1], fb0, P0[-PHX], fap1, fam1, ua - mu_, uax - mu_, va - mv_, v_b, wa0 - mw_,
+               waz - mw_, ((Fx[1] - Fx[-1]) + (yb0 - Fy[-PHX])) + (zap1 - zam1), roa);
+      out_cell(c + nx, fb0, P0[PHX + 1], P0[PHX - 1], P0[2 * PHX], fa0, fbp1, fbm1, ub - mu_, ubx - mu_, v_b, vc - mv_,
+               wb0 - mw_, wbz - mw_, ((Fx[PHX + 1] - Fx[PHX - 1]) + (Fy[2 * PHX] - ya0)) + (zbp1 - zbm1), rob);
+      wa0 = waz;
+      wb0 = wbz;
       c += plane;
     }
+    __pipeline_wait_prior(0);
     __syncthreads();
-    f_m1 = f_0;
-    f_0 = f_p1;
-    f_p1 = f_p2;
-    f_p2 = f_p3;
-    s_0 = s_p1;
-    s_p1 = s_p2;
-    z_m1 = z_0;
-    z_0 = z_p1;
+    fam1 = fa0, fa0 = fap1, fap1 = fap2, fap2 = fap3;
+    fbm1 = fb0, fb0 = fbp1, fbp1 = fbp2, fbp2 = fbp3;
+    sa0 = sap1, sap1 = sap2, sb0 = sbp1, sbp1 = sbp2;
+    zam1 = za0, za0 = zap1, zbm1 = zb0, zb0 = zbp1;
+    ya0 = yap1, yb0 = ybp1;
   };
   // k0 and the chunk are even (launch_phase), so k0 - 4 is even and the trip count too; two
-  // planes per iteration, four per unrolled body (2.58 ms at 512^3 with runtime slots, against
-  // 2.67 for two, 2.69 for one and 2.60 for eight planes, where it spills); the same bits for
-  // every unroll factor
-#pragma unroll 2
+  // planes per iteration
+#pragma unroll PUNROLL
   for (int k = k0 - 4; k < k1; k += 2) {
     plane_iter(std::integral_constant<int, 0>{}, k);
     plane_iter(std::integral_constant<int, 1>{}, k + 1);
@@ -284,8 +361,9 @@ int phase_zchunk(const Geo& g, int requested, bool many) {
   }
   // The even chunk with the fewest planes in sequence on an SM: waves of one block on each of the
   // 148 SMs times the chunk with its four planes of warm-up (the shorter list of chunks on a tie).
-  // Measured, chunk of 64 -> the rule's: 128^3 87 -> 50 us (32 planes), 192x64x128 83 -> 37 us
-  // (22 planes), 256^3 345 -> 321 us (256 planes); 512^3 takes 256 planes (2.27 ms; 2.31 with 128).
+  // With the 32 x 16 tiles of before and chunks of 64, then of the rule: 128^3 87 -> 50 us (32
+  // planes), 192x64x128 83 -> 37 us (22), 256^3 345 -> 331 us (32); with the 32 x 24 tiles 45 us
+  // (22), 36 us (16) and 254 us (52), 512^3 104 planes.
   // Results do not depend on the chunk.
   return best_zchunk(g.nz, cols, 148, 4);
 }
@@ -295,7 +373,7 @@ dim3 phase_grid(const Geo& g, int zc) {
 }
 
 cudaError_t launch_phase_batch(const BatchArgs<PhaseArgs>& b, bool clamp, int nsm, cudaStream_t st) {
-  constexpr size_t smem = 8 * sizeof(double) * PNT;
+  constexpr size_t smem = PSMEM;
   auto kern = clamp ? k_phase_batch<true> : k_phase_batch<false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
@@ -306,7 +384,7 @@ cudaError_t launch_phase_batch(const BatchArgs<PhaseArgs>& b, bool clamp, int ns
 }
 
 cudaError_t launch_phase(const PhaseArgs& a, cudaStream_t st) {
-  constexpr size_t smem = 8 * sizeof(double) * PNT;  // psi, phi, Fx, Fy: two planes each
+  constexpr size_t smem = PSMEM;
   auto kern = a.clamp ? k_phase<true> : k_phase<false>;
   static int attr_set[64][2] = {};
   int dev = 0;
