@@ -223,41 +223,74 @@ cudaError_t launch_finalize(const double* partials, int nblocks, const Geo& g, D
 // max |div u| (the operator of :841-843 without rho/dt), kinetic energy, and the dissipation
 // 2 nu <S_ij S_ij> with central differences (post/compute_diss/main.f90:72-117).  The maximum
 // propagates NaN, so a NaN velocity gives a NaN max|div| as well as a NaN KE.
-__global__ void __launch_bounds__(CNT) k_diag(DiagArgs a) {
+//
+// The tiles and threads of k_correct: each thread owns two adjacent x cells of a tile row and
+// marches up the chunk with the planes k-1, k, k+1 of its pair in registers, so a plane costs it
+// one 16-byte load per field (k+1), the two rows beside it and the two cells beside the pair, which
+// L1 serves: 7.5 loads per cell.  One cell per thread with its 25 loads and the 64-bit divisions
+// of its index took 2.80 ms at 512^3; the compulsory 24 bytes per cell take 0.49 ms.
+struct DiagPair {
+  double2 m, c, p;  // planes k-1, k, k+1 of the thread's pair
+};
+__global__ void __launch_bounds__(CNT) k_diag(DiagArgs a, int zc) {
   const Geo& g = a.g;
   const int nx = g.nx, ny = g.ny, nz = g.nz;
-  const size_t ntot = (size_t)nx * ny * nz;
-  const double mu_ = a.sc->mean[0], mv_ = a.sc->mean[1], mw_ = a.sc->mean[2];
-  const double* __restrict__ U = a.u;
-  const double* __restrict__ V = a.v;
-  const double* __restrict__ W = a.w;
+  const size_t plane = (size_t)nx * ny;
   const double dxi = g.dxi, h = 0.5 / a.dxd;
+  const double* const fld[3] = {a.u, a.v, a.w};
+  const double mean[3] = {a.sc->mean[0], a.sc->mean[1], a.sc->mean[2]};
+  const int lx = threadIdx.x & 15, ty = threadIdx.x >> 4;  // 16 lanes x 16 rows
+  const int i = blockIdx.x * CTX + 2 * lx, j = blockIdx.y * CTY + ty;
+  const int k0 = blockIdx.z * zc, k1 = min(k0 + zc, nz);
   double mdiv = 0.0, ke = 0.0, ss = 0.0;
-  const size_t stride = (size_t)gridDim.x * CNT;
-  for (size_t c = (size_t)blockIdx.x * CNT + threadIdx.x; c < ntot; c += stride) {
-    const int i = (int)(c % nx);
-    const size_t r = c / nx;
-    const int j = (int)(r % ny), k = (int)(r / ny);
-    const int ip = wrapp(i, nx), im = wrapm(i, nx), jp = wrapp(j, ny), jm = wrapm(j, ny);
-    const int kp = wrapp(k, nz), km = wrapm(k, nz);
-#define F(A, m, ii, jj, kk) (__ldg(A + lin(ii, jj, kk, nx, ny)) - m)
-    const double u0 = F(U, mu_, i, j, k), v0 = F(V, mv_, i, j, k), w0 = F(W, mw_, i, j, k);
-    const double div = (F(U, mu_, ip, j, k) - u0) * dxi + (F(V, mv_, i, jp, k) - v0) * dxi +
-                       (F(W, mw_, i, j, kp) - w0) * dxi;
-    mdiv = nanmax(mdiv, fabs(div));
-    ke += u0 * u0 + v0 * v0 + w0 * w0;
-    const double dudx = (F(U, mu_, ip, j, k) - F(U, mu_, im, j, k)) * h;
-    const double dudy = (F(U, mu_, i, jp, k) - F(U, mu_, i, jm, k)) * h;
-    const double dudz = (F(U, mu_, i, j, kp) - F(U, mu_, i, j, km)) * h;
-    const double dvdx = (F(V, mv_, ip, j, k) - F(V, mv_, im, j, k)) * h;
-    const double dvdy = (F(V, mv_, i, jp, k) - F(V, mv_, i, jm, k)) * h;
-    const double dvdz = (F(V, mv_, i, j, kp) - F(V, mv_, i, j, km)) * h;
-    const double dwdx = (F(W, mw_, ip, j, k) - F(W, mw_, im, j, k)) * h;
-    const double dwdy = (F(W, mw_, i, jp, k) - F(W, mw_, i, jm, k)) * h;
-    const double dwdz = (F(W, mw_, i, j, kp) - F(W, mw_, i, j, km)) * h;
-#undef F
-    const double s12 = 0.5 * (dudy + dvdx), s13 = 0.5 * (dudz + dwdx), s23 = 0.5 * (dvdz + dwdy);
-    ss += dudx * dudx + dvdy * dvdy + dwdz * dwdz + 2.0 * (s12 * s12 + s13 * s13 + s23 * s23);
+  if (i < nx && j < ny) {
+    const int im = wrapm(i, nx), ip = wrapp(i + 1, nx), jm = wrapm(j, ny), jp = wrapp(j, ny);
+    const size_t r0 = (size_t)j * nx, rm = (size_t)jm * nx, rp = (size_t)jp * nx;
+    auto pair = [&](int f, size_t o) {
+      const double2 v = __ldg(reinterpret_cast<const double2*>(fld[f] + o));
+      return make_double2(v.x - mean[f], v.y - mean[f]);
+    };
+    DiagPair q[3];
+#pragma unroll
+    for (int f = 0; f < 3; ++f) {
+      q[f].c = pair(f, (size_t)wrapm(k0, nz) * plane + r0 + i);
+      q[f].p = pair(f, (size_t)k0 * plane + r0 + i);
+    }
+    for (int k = k0; k < k1; ++k) {
+      const size_t pk = (size_t)k * plane, pp = (size_t)wrapp(k, nz) * plane;
+      double xm[3], xp[3];        // the cells left and right of the pair
+      double2 ym[3], yp[3];       // the rows below and above
+#pragma unroll
+      for (int f = 0; f < 3; ++f) {
+        q[f].m = q[f].c;
+        q[f].c = q[f].p;
+        q[f].p = pair(f, pp + r0 + i);
+        ym[f] = pair(f, pk + rm + i);
+        yp[f] = pair(f, pk + rp + i);
+        xm[f] = __ldg(fld[f] + pk + r0 + im) - mean[f];
+        xp[f] = __ldg(fld[f] + pk + r0 + ip) - mean[f];
+      }
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {  // the two cells
+        double c0[3], dx[3], dy[3], dz[3], fx, fy, fz;
+#pragma unroll
+        for (int f = 0; f < 3; ++f) {
+          const double vx = e ? xp[f] : q[f].c.y, vw = e ? q[f].c.x : xm[f];
+          c0[f] = e ? q[f].c.y : q[f].c.x;
+          dx[f] = (vx - vw) * h;
+          dy[f] = ((e ? yp[f].y : yp[f].x) - (e ? ym[f].y : ym[f].x)) * h;
+          dz[f] = ((e ? q[f].p.y : q[f].p.x) - (e ? q[f].m.y : q[f].m.x)) * h;
+          if (f == 0) fx = vx;
+          if (f == 1) fy = e ? yp[f].y : yp[f].x;
+          if (f == 2) fz = e ? q[f].p.y : q[f].p.x;
+        }
+        const double div = (fx - c0[0]) * dxi + (fy - c0[1]) * dxi + (fz - c0[2]) * dxi;
+        mdiv = nanmax(mdiv, fabs(div));
+        ke += c0[0] * c0[0] + c0[1] * c0[1] + c0[2] * c0[2];
+        const double s12 = 0.5 * (dy[0] + dx[1]), s13 = 0.5 * (dz[0] + dx[2]), s23 = 0.5 * (dz[1] + dy[2]);
+        ss += dx[0] * dx[0] + dy[1] * dy[1] + dz[2] * dz[2] + 2.0 * (s12 * s12 + s13 * s13 + s23 * s23);
+      }
+    }
   }
   __shared__ double red[3][CNT / 32];
   double vals[3] = {mdiv, ke, ss};
@@ -276,7 +309,8 @@ __global__ void __launch_bounds__(CNT) k_diag(DiagArgs a) {
     const int q = threadIdx.x;
     double x = red[q][0];
     for (int wv = 1; wv < CNT / 32; ++wv) x = q == 0 ? nanmax(x, red[q][wv]) : x + red[q][wv];
-    a.partials[(size_t)blockIdx.x * 4 + q] = x;
+    const size_t bid = ((size_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+    a.partials[bid * 4 + q] = x;
   }
 }
 
@@ -316,10 +350,10 @@ __global__ void __launch_bounds__(1024) k_diag_finalize(const double* __restrict
 }
 
 cudaError_t launch_diag(const DiagArgs& a, cudaStream_t st) {
-  k_diag<<<a.nblocks, CNT, 0, st>>>(a);
+  k_diag<<<correct_grid(a.g), CNT, 0, st>>>(a, correct_chunk(a.g));
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  k_diag_finalize<<<1, 1024, 0, st>>>(a.partials, a.nblocks, a.g, a.nu, a.sc);
+  k_diag_finalize<<<1, 1024, 0, st>>>(a.partials, correct_blocks(a.g), a.g, a.nu, a.sc);
   return cudaGetLastError();
 }
 

@@ -170,8 +170,7 @@ int xc_blocks(const Geo& g, int zc);
 struct DiagArgs {
   Geo g;
   const double *u, *v, *w;
-  double* partials;  // [nblocks][4]
-  int nblocks;
+  double* partials;  // [correct_blocks(g)][4]
   DevScalars* sc;
   double nu, dxd;    // viscosity and spacing used by the dissipation formula
 };
@@ -211,8 +210,8 @@ struct LabelArgs {
   long long bound = 0;          // iteration bound of the union-find loops (0: the cell count)
 };
 int label_chunks(int n);
-cudaError_t launch_label_components(const LabelArgs& a, cudaStream_t st);  // init, merge, flatten, count
-cudaError_t launch_label_number(const LabelArgs& a, cudaStream_t st);      // counts must hold offsets
+cudaError_t launch_label_components(const LabelArgs& a, cudaStream_t st);  // init, merge, flatten and count
+cudaError_t launch_label_number(const LabelArgs& a, cudaStream_t st);      // counts must hold offsets and the total
 cudaError_t launch_label_stats(const LabelArgs& a, cudaStream_t st);
 
 // ---------------------------------------------------------------- initial conditions

@@ -75,6 +75,8 @@ struct mhit_ctx {
   void *twx = nullptr, *twy = nullptr, *twz = nullptr;
   void* spec64 = nullptr;  // energy spectrum in the FP32 modes: an FP64 half spectrum, grown lazily
   size_t spec64_bytes = 0;
+  void* spec_acc = nullptr;  // energy spectrum: shell sums and the blocks' histograms, grown lazily
+  size_t spec_acc_bytes = 0;
   void* tw64[3] = {};      // ... and FP64 twiddles
   double *k2x = nullptr, *k2y = nullptr, *k2z = nullptr;
   double* tabs = nullptr;
@@ -586,6 +588,7 @@ void mhit_destroy(mhit_ctx* c) {
   cudaFree(c->lab_acc);
   cudaFree(c->spec);
   cudaFree(c->spec64);
+  cudaFree(c->spec_acc);
   for (void* t : c->tw64) cudaFree(t);
   cudaFree(c->twx);
   cudaFree(c->twy);
@@ -963,7 +966,6 @@ int mhit_diagnostics(mhit_ctx* c, mhit_diag* d) {
   a.v = c->V[c->cur];
   a.w = c->W[c->cur];
   a.partials = c->partials;
-  a.nblocks = c->nblk;
   a.sc = c->sc;
   a.nu = c->prm.mu / c->prm.rho;
   a.dxd = c->g.dx;
@@ -1270,7 +1272,8 @@ int mhit_label_drops(mhit_ctx* c, double thresh, int connectivity, mhit_drop* dr
     cnt[b] = total;
     total += k;
   }
-  MHIT_CUDA_TRY(cudaMemcpyAsync(counts, cnt.data(), sizeof(int) * nch, cudaMemcpyHostToDevice, c->st));
+  cnt[nch] = total;  // over the error flag, read above
+  MHIT_CUDA_TRY(cudaMemcpyAsync(counts, cnt.data(), sizeof(int) * (nch + 1), cudaMemcpyHostToDevice, c->st));
   MHIT_CUDA_TRY(launch_label_number(a, c->st));
   const size_t nd = (size_t)std::max(total, 1);
   const size_t acc_bytes = nd * (9 * sizeof(double) + sizeof(unsigned long long));
@@ -1476,10 +1479,11 @@ int mhit_energy_spectrum(mhit_ctx* c, double* E, int nbins) {
     ty = c->tw64[1];
     tz = c->tw64[2];
   }
-  DevBuf dpart, dE;
-  MHIT_CUDA_TRY(cudaMalloc(&dpart.p, (size_t)spectrum_blocks(g) * nbins * sizeof(double)));
-  MHIT_CUDA_TRY(cudaMalloc(&dE.p, (size_t)nbins * sizeof(double)));
-  MHIT_CUDA_TRY(cudaMemsetAsync(dE.p, 0, (size_t)nbins * sizeof(double), c->st));
+  // the shell sums, then every block's histogram
+  if ((rc = grow_buffer(&c->spec_acc, &c->spec_acc_bytes, ((size_t)spectrum_blocks(g) + 1) * nbins * sizeof(double))))
+    return rc;
+  double* dE = static_cast<double*>(c->spec_acc);
+  MHIT_CUDA_TRY(cudaMemsetAsync(dE, 0, (size_t)nbins * sizeof(double), c->st));
   const double* fields[3] = {c->U[c->cur], c->V[c->cur], c->W[c->cur]};
   for (int comp = 0; comp < 3; ++comp) {
     PoissonArgs a;
@@ -1500,9 +1504,9 @@ int mhit_energy_spectrum(mhit_ctx* c, double* E, int nbins) {
     MHIT_CUDA_TRY(poisson_stage(a, PSTAGE_YFWD, c->st));
     MHIT_CUDA_TRY(poisson_stage(a, PSTAGE_ZFWD, c->st));
     MHIT_CUDA_TRY(launch_spectrum_bin(static_cast<const Cx<double>*>(spec), g, c->sc, comp, nbins,
-                                      static_cast<double*>(dpart.p), static_cast<double*>(dE.p), c->st));
+                                      dE + nbins, dE, c->st));
   }
-  MHIT_CUDA_TRY(cudaMemcpyAsync(E, dE.p, (size_t)nbins * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+  MHIT_CUDA_TRY(cudaMemcpyAsync(E, dE, (size_t)nbins * sizeof(double), cudaMemcpyDeviceToHost, c->st));
   MHIT_CUDA_TRY(cudaStreamSynchronize(c->st));
   return MHIT_OK;
 }
