@@ -5,7 +5,9 @@
 // k_finalize    one block reduces the partials in a fixed order (run-to-run deterministic),
 //               writes mean = sum/nx/ny/nz (:967-969), gumax = max over components of
 //               (max - mean) -- equal to maxval(u - mean) because rounding is monotonic --,
-//               cfl = gumax dt dxi (:1003) and the NaN / CFL>7 flags (:1006).
+//               cfl = gumax dt dxi (:1003) and the NaN / CFL>7 flags (:1006), and copies the
+//               scalars to the host's page-locked copy: a host that looks at every step waits for
+//               the stream only, without a copy of 128 bytes behind each step (SC_MEASURED).
 // The mean is not subtracted here: the next step's kernels and the download subtract it on
 // read, which saves a full read+write pass of u, v, w.
 #include "common.cuh"
@@ -135,7 +137,7 @@ __global__ void __launch_bounds__(CNT) k_correct(CorrectArgs a, S ps, int zc) {
 }
 
 __global__ void __launch_bounds__(1024) k_finalize(const double* __restrict__ partials, int nblocks, Geo g,
-                                                   DevScalars* sc) {
+                                                   DevScalars* sc, DevScalars* host) {
   __shared__ double red[6][32];
   double vals[6] = {0.0, 0.0, 0.0, -INFINITY, -INFINITY, -INFINITY};
   for (int b = threadIdx.x; b < nblocks; b += blockDim.x) {
@@ -178,6 +180,7 @@ __global__ void __launch_bounds__(1024) k_finalize(const double* __restrict__ pa
     if (!(gumax == gumax)) flag |= 1;
     if (sc->cfl > 7.0) flag |= 2;  // :1006
     sc->flag |= flag;
+    if (host) *host = *sc;
   }
 }
 
@@ -211,11 +214,12 @@ cudaError_t launch_correct(const CorrectArgs& a, cudaStream_t st) {
   else k_correct<<<grd, blk, 0, st>>>(a, PDouble{static_cast<const double*>(a.p)}, zc);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  return launch_finalize(a.partials, a.nblocks, a.g, a.sc, st);
+  return launch_finalize(a.partials, a.nblocks, a.g, a.sc, a.sc_host, st);
 }
 
-cudaError_t launch_finalize(const double* partials, int nblocks, const Geo& g, DevScalars* sc, cudaStream_t st) {
-  k_finalize<<<1, 1024, 0, st>>>(partials, nblocks, g, sc);
+cudaError_t launch_finalize(const double* partials, int nblocks, const Geo& g, DevScalars* sc, DevScalars* host,
+                            cudaStream_t st) {
+  k_finalize<<<1, 1024, 0, st>>>(partials, nblocks, g, sc, host);
   return cudaGetLastError();
 }
 

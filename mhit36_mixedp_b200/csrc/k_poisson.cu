@@ -340,7 +340,12 @@ template <typename T, int N, int MODE> struct ColTile {
   static constexpr bool Z64 = MODE == 2 && N == 512 && sizeof(T) == 8;
   static constexpr int B = Z64 ? 4 : 8;
   static constexpr int NT = Z64 ? fft_threads<N, 4>() : ColSched<T, N, MODE>::NT;
-  static constexpr int MINB = Z64 ? 2 : ((MODE == 2 && sizeof(T) == 8) ? 1 : ColSched<T, N, MODE>::MINB);
+  // FP64 single transforms of 256 points (radix 16 x 16, 128 threads): at 128 registers four blocks
+  // fit an SM without spilling, against two at the 194 the compiler takes unbounded: y passes
+  // 57.7 -> 48 us at 256^3 (five blocks spill: 60 us)
+  static constexpr bool Y64 = MODE != 2 && N == 256 && sizeof(T) == 8;
+  static constexpr int MINB =
+      Z64 ? 2 : (Y64 ? 4 : ((MODE == 2 && sizeof(T) == 8) ? 1 : ColSched<T, N, MODE>::MINB));
   using S = typename ColSched<T, N, MODE>::S;
 };
 

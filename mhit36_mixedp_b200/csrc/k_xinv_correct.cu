@@ -417,7 +417,7 @@ static cudaError_t launch_xc_m(const XcArgs& a, cudaStream_t st) {
   kern<<<grid, NT, smem, st>>>(b);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  return launch_finalize(a.partials, (int)(grid.x * grid.y), a.g, a.sc, st);
+  return launch_finalize(a.partials, (int)(grid.x * grid.y), a.g, a.sc, a.sc_host, st);
 }
 
 template <typename T>

@@ -141,11 +141,14 @@ struct CorrectArgs {
   double* partials;   // [nblocks][6]
   int nblocks;
   DevScalars* sc;
+  DevScalars* sc_host = nullptr;  // page-locked host copy, written with sc
 };
 cudaError_t launch_correct(const CorrectArgs& a, cudaStream_t st);
 int correct_blocks(const Geo& g);
-// k_finalize: the projection's partial sums/maxima -> mean, gumax, cfl, flags (fixed order)
-cudaError_t launch_finalize(const double* partials, int nblocks, const Geo& g, DevScalars* sc, cudaStream_t st);
+// k_finalize: the projection's partial sums/maxima -> mean, gumax, cfl, flags (fixed order); host:
+// a page-locked copy of sc to write as well, or null
+cudaError_t launch_finalize(const double* partials, int nblocks, const Geo& g, DevScalars* sc, DevScalars* host,
+                            cudaStream_t st);
 
 // the inverse x transform fused with the projection (the pressure stays on chip): u*, v*, w*
 // projected in place from the y-inverted spectrum, partial sums/maxima as k_correct, then
@@ -161,6 +164,7 @@ struct XcArgs {
   float* qnew = nullptr;
   double* partials;           // [xc_blocks(g)][6]
   DevScalars* sc;
+  DevScalars* sc_host = nullptr;  // page-locked host copy, written with sc
   int zc = 0;                 // z planes per block (0: default)
 };
 cudaError_t launch_xinv_correct(const XcArgs& a, cudaStream_t st);

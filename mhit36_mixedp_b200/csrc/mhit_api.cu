@@ -352,6 +352,7 @@ static int enqueue_stage(mhit_ctx* c, int stage, double alpha, double beta, int 
         }
         x.partials = c->partials;
         x.sc = c->sc;
+        x.sc_host = c->sc_host;
         MHIT_CUDA_TRY(launch_xinv_correct(x, c->st));
         return MHIT_OK;
       }
@@ -366,6 +367,7 @@ static int enqueue_stage(mhit_ctx* c, int stage, double alpha, double beta, int 
       a.partials = c->partials;
       a.nblocks = c->nblk;
       a.sc = c->sc;
+      a.sc_host = c->sc_host;
       MHIT_CUDA_TRY(launch_correct(a, c->st));
       return MHIT_OK;
     }
@@ -466,6 +468,7 @@ static int enqueue_steps(mhit_ctx* c, int nsteps) {
   return MHIT_OK;
 }
 
+// the device scalars into sc_host; after a step the projection has already written them there
 static int fetch_scalars(mhit_ctx* c) {
   MHIT_CUDA_TRY(cudaMemcpyAsync(c->sc_host, c->sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, c->st));
   MHIT_CUDA_TRY(cudaStreamSynchronize(c->st));
@@ -853,7 +856,8 @@ int mhit_step(mhit_ctx* c, int nsteps) {
   if ((rc = check_ctx(c))) return rc;
   if (nsteps < 0) return set_error(MHIT_ERR_ARG, "nsteps < 0");
   if ((rc = enqueue_steps(c, nsteps))) return rc;
-  if ((rc = fetch_scalars(c))) return rc;
+  if (nsteps > 0) MHIT_CUDA_TRY(cudaStreamSynchronize(c->st));
+  else if ((rc = fetch_scalars(c))) return rc;
   if (c->sc_host->flag & 4)
     return set_error(MHIT_ERR_TIMEOUT, "the tensor-core z solve gave up on a bounded wait (results invalid)");
   if (c->sc_host->flag & 1) return set_error(MHIT_ERR_NAN, "NaN in the velocity field");
@@ -1880,11 +1884,11 @@ static int ens_enqueue_steps(mhit_ensemble* e, int nsteps) {
   return MHIT_OK;
 }
 
-static int ens_check_flags(mhit_ensemble* e) {
+static int ens_check_flags(mhit_ensemble* e, bool stepped) {
   MHIT_CUDA_TRY(cudaStreamSynchronize(e->st));
   for (int b = 0; b < e->nbox; ++b) {
     int rc;
-    if ((rc = fetch_scalars(e->box[b]))) return rc;
+    if (!stepped && (rc = fetch_scalars(e->box[b]))) return rc;
     const int flag = e->box[b]->sc_host->flag;
     if (flag & 1) return set_error(MHIT_ERR_NAN, "NaN in the velocity field of ensemble box " + std::to_string(b));
     if (flag & 2) return set_error(MHIT_ERR_CFL, "CFL > 7 in ensemble box " + std::to_string(b));
@@ -1975,7 +1979,7 @@ int mhit_ensemble_step(mhit_ensemble* e, int nsteps) {
   for (mhit_ctx* c : e->box) MHIT_CUDA_TRY(cudaStreamSynchronize(c->st));
   int rc;
   if ((rc = ens_enqueue_steps(e, nsteps))) return rc;
-  return ens_check_flags(e);
+  return ens_check_flags(e, nsteps > 0);
 }
 
 int mhit_ensemble_time_steps(mhit_ensemble* e, int nsteps, double* ms) {
