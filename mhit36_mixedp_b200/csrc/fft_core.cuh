@@ -311,18 +311,26 @@ __device__ __forceinline__ void st_read(const Cx<T>* s, Cx<T> (&a)[StageShape<N,
   }
 }
 
+// Multiplies operand r of butterfly t by exp(-+ 2 pi i r k / (p R)), k = t mod p, and transforms.  The
+// factors lie stage by stage as tws[r - 1][k] (axis_twiddles), so the lanes of a warp (consecutive
+// t) read neighbouring entries: indexed r k L/(p R) into one table of exp(-2 pi i m / L), a warp's
+// load touched up to eight 128-byte lines, and these loads were a third of the shared-memory and L1
+// wavefronts of a column pass.  The same factors, the same bits: at 512^3 the FP32 z solve 606 -> 506
+// us, the FP32 y passes 224 / 234 -> 213 us, the FP64 column passes unchanged (their 16-byte factors
+// are a smaller share, and the latency of the FP64 chains bounds them).  The transforms staged through
+// shared memory (stockham_stage) keep the one table: with the ordered one the FP32 x pass took 123
+// instead of 113 us at 256^3.
 template <typename T, int N, int B, int NT, int R, bool INV>
-__device__ __forceinline__ void st_compute(Cx<T> (&a)[StageShape<N, B, NT, R>::BPT][R], const Cx<T>* __restrict__ tw,
-                                           int twstride, int p) {
+__device__ __forceinline__ void st_compute(Cx<T> (&a)[StageShape<N, B, NT, R>::BPT][R], const Cx<T>* __restrict__ tws,
+                                           int p) {
 #pragma unroll
   for (int m = 0; m < StageShape<N, B, NT, R>::BPT; ++m) {
     if (st_valid<N, B, NT, R>(m)) {
       const int q = threadIdx.x + m * NT, t = q / B, k = t % p;
       if (p > 1) {
-        const int step = (N / (p * R)) * twstride;
 #pragma unroll
         for (int r = 1; r < R; ++r) {
-          Cx<T> w = tw[r * k * step];
+          Cx<T> w = tws[(r - 1) * p + k];
           if (INV) w.y = -w.y;
           a[m][r] = cmul(a[m][r], w);
         }
@@ -345,18 +353,19 @@ __device__ __forceinline__ void st_write(Cx<T>* s, const Cx<T> (&a)[StageShape<N
   }
 }
 
-// Full transform in radix order REV: `in` holds the first stage's operands (elements
+// Full transform in radix order REV with that order's stage twiddles tws (the stage after radices of
+// product p starts at p - R_0, a telescoping sum): `in` holds the first stage's operands (elements
 // t + r N/R0), `out` receives the last stage's results (elements t + r N/R_last).  s is used
 // between stages; on entry no thread may still be reading s, and on return threads may still
 // be reading it (the caller synchronises before writing s again).
 template <typename T, int N, int B, int NT, bool INV, bool REV, typename S = Radix<N>>
 __device__ __forceinline__ void fft_regs(
-    Cx<T>* s, const Cx<T>* __restrict__ tw, int twstride,
+    Cx<T>* s, const Cx<T>* __restrict__ tws,
     Cx<T> (&in)[StageShape<N, B, NT, srad<S, REV>(0)>::BPT][srad<S, REV>(0)],
     Cx<T> (&out)[StageShape<N, B, NT, srad<S, REV>(S::ns - 1)>::BPT][srad<S, REV>(S::ns - 1)]) {
   constexpr int NS = S::ns;
   constexpr int R0 = srad<S, REV>(0);
-  st_compute<T, N, B, NT, R0, INV>(in, tw, twstride, 1);
+  st_compute<T, N, B, NT, R0, INV>(in, tws, 1);
   if constexpr (NS == 1) {
 #pragma unroll
     for (int m = 0; m < StageShape<N, B, NT, R0>::BPT; ++m)
@@ -370,13 +379,13 @@ __device__ __forceinline__ void fft_regs(
       Cx<T> a1[StageShape<N, B, NT, R1>::BPT][R1];
       st_read<T, N, B, NT, R1>(s, a1);
       __syncthreads();
-      st_compute<T, N, B, NT, R1, INV>(a1, tw, twstride, spbefore<S, REV>(1));
+      st_compute<T, N, B, NT, R1, INV>(a1, tws, R0);
       st_write<T, N, B, NT, R1>(s, a1, spbefore<S, REV>(1));
       __syncthreads();
     }
     constexpr int RL = srad<S, REV>(NS - 1);
     st_read<T, N, B, NT, RL>(s, out);
-    st_compute<T, N, B, NT, RL, INV>(out, tw, twstride, spbefore<S, REV>(NS - 1));
+    st_compute<T, N, B, NT, RL, INV>(out, tws + (spbefore<S, REV>(NS - 1) - R0), spbefore<S, REV>(NS - 1));
   }
 }
 

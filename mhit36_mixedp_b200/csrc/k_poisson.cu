@@ -15,6 +15,7 @@
 #include <cuda_pipeline.h>
 
 #include <type_traits>
+#include <vector>
 
 #include "common.cuh"
 #include "fft_core.cuh"
@@ -345,7 +346,9 @@ template <typename T, int N, int MODE> struct ColTile {
   // 57.7 -> 48 us at 256^3 (five blocks spill: 60 us)
   static constexpr bool Y64 = MODE != 2 && N == 256 && sizeof(T) == 8;
   static constexpr int MINB =
-      Z64 ? 2 : (Y64 ? 4 : ((MODE == 2 && sizeof(T) == 8) ? 1 : ColSched<T, N, MODE>::MINB));
+      Z64 ? 2
+          : (Y64 ? 4 : (MODE != 2 ? ColSched<T, N, MODE>::MINB
+                                  : (sizeof(T) == 8 ? 1 : (N == 256 ? 3 : ColSched<T, N, MODE>::MINB))));
   using S = typename ColSched<T, N, MODE>::S;
 };
 
@@ -378,7 +381,7 @@ k_fft_cols(Cx<T>* __restrict__ spec, const Cx<T>* __restrict__ tw, Geo g, size_t
     }
   }
   Cx<T> z[BL][RL];
-  fft_regs<T, N, B, NT, MODE == 1, false, S>(s, tw, 1, a, z);
+  fft_regs<T, N, B, NT, MODE == 1, false, S>(s, tw + N, a, z);
   if constexpr (MODE == 2) {
     // multi/main.f90:889-895: phi3d = -phi3d/k2/(nx*ny*nz) in FP64, phi3d(1,1,1) = 0.
     // One reciprocal of k2*N per element (within 2 ulp of the reference's two divides).
@@ -403,7 +406,7 @@ k_fft_cols(Cx<T>* __restrict__ spec, const Cx<T>* __restrict__ tw, Geo g, size_t
       }
     }
     __syncthreads();  // every thread has read the forward transform's last stage
-    fft_regs<T, N, B, NT, true, true, S>(s, tw, 1, z, a);
+    fft_regs<T, N, B, NT, true, true, S>(s, tw + 2 * N, z, a);
 #pragma unroll
     for (int m = 0; m < BA; ++m) {
       if (st_valid<N, B, NT, RA>(m)) {
@@ -429,7 +432,7 @@ k_fft_cols(Cx<T>* __restrict__ spec, const Cx<T>* __restrict__ tw, Geo g, size_t
 }
 // The same passes with the whole tile staged in shared memory (cp.async in, every stage
 // through shared memory, stores from shared memory): fewer registers per thread, which wins for
-// the short transforms whose register-staged version needs 16-point butterflies.
+// the FP64 256-point z solve, whose register-staged version holds 16-point butterflies.
 template <typename T, int N, int MODE>
 __global__ void __launch_bounds__(fft_threads<N, Tile<T>::B>())
 k_fft_cols_smem(Cx<T>* __restrict__ spec, const Cx<T>* __restrict__ tw, Geo g, size_t stride_n,
@@ -514,9 +517,9 @@ static cudaError_t launch_xinv_m(const PoissonArgs& a, cudaStream_t st) {
 
 template <typename T, int N, int MODE>
 static cudaError_t launch_cols_n(const PoissonArgs& a, int axis, cudaStream_t st) {
-  // the 256-point z solve runs faster staged in shared memory (measured at 256^3: 0.066 vs
-  // 0.072 ms FP32, 0.105 vs 0.117 ms FP64); every other pass and size register-staged
-  constexpr bool staged = MODE == 2 && N == 256;
+  // the FP64 256-point z solve runs faster staged in shared memory (measured at 256^3: 0.105 vs
+  // 0.113 ms; FP32, three blocks per SM: 0.066 vs 0.064 ms); every other pass and size register-staged
+  constexpr bool staged = MODE == 2 && N == 256 && sizeof(T) == 8;
   constexpr int B = staged ? Tile<T>::B : ColTile<T, N, MODE>::B;
   constexpr int NT = staged ? fft_threads<N, B>() : ColTile<T, N, MODE>::NT;
   const size_t smem = (size_t)N * B * sizeof(Cx<T>);
@@ -565,6 +568,27 @@ static cudaError_t launch_cols(const PoissonArgs& a, int axis, cudaStream_t st) 
 #undef C
   }
   return cudaErrorInvalidValue;
+}
+
+template <typename S> static std::vector<int> radices() {
+  std::vector<int> v;
+  for (int i = 0; i < S::ns; ++i) {
+    const int q[3] = {S::r[0], S::r[1], S::r[2]};
+    v.push_back(q[i]);
+  }
+  return v;
+}
+
+std::vector<int> fft_schedule(int n, int axis, bool fp32) {
+  switch (n) {
+#define C(m)                                                                                                \
+  case m:                                                                                                   \
+    return axis == 1 ? (fp32 ? radices<ColSched<float, m, 0>::S>() : radices<ColSched<double, m, 0>::S>())  \
+                     : (fp32 ? radices<ColSched<float, m, 2>::S>() : radices<ColSched<double, m, 2>::S>());
+    MHIT_NSIZES(C)
+#undef C
+  }
+  return {};
 }
 
 bool poisson_size_supported(int n, bool is_x) {

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <string>
+#include <vector>
 
 #include "../../include/mhit_b200.h"
 #include "common.cuh"
@@ -32,7 +33,9 @@ struct PoissonArgs {
   const double *u, *v, *w;  // u* (input of the divergence)
   void* spec;               // Cx<T>[nz][ny][pitch]
   void* p;                  // T[nz][ny][nx]
-  const void *twx, *twy, *twz;  // exp(-2 pi i m/n) tables, one per axis, in T
+  // exp(-2 pi i m/n) tables, one per axis, in T; those of y and z are followed by the stage twiddles
+  // of the axis's radix schedule (axis_twiddles)
+  const void *twx, *twy, *twz;
   const double *k2x, *k2y, *k2z;
   double cdiv;  // rho*dxi/dt
   double ntot;  // nx*ny*nz
@@ -56,6 +59,8 @@ cudaError_t launch_zsolve_tc(const ZsolveTc* z, const PoissonArgs& a, DevScalars
 cudaError_t launch_combine(const float* p32, const float* d32, double* p64, size_t n, cudaStream_t st);
 cudaError_t poisson_stage(const PoissonArgs& a, int stage, cudaStream_t st);
 bool poisson_size_supported(int n, bool is_x);
+// radices of the transform along y (axis 1) or z (axis 2) of n points, in stage order
+std::vector<int> fft_schedule(int n, int axis, bool fp32);
 
 // z planes per block of a stencil that marches `cols` columns of nz planes on `slots` resident
 // blocks and spends `warm` planes' time at the start of each chunk: the even chunk with the least

@@ -151,6 +151,32 @@ static std::vector<T> twiddles(int n) {
   return t;
 }
 
+// The table exp(-2 pi i m/n) of the y (1) or z (2) axis and behind it, from entry n, the stage
+// twiddles of its radix schedule: exp(-2 pi i r k/(p R)) as [r - 1][k] for every stage of radix R after
+// stages of product p > 1; then the same for the reversed order, from entry 2 n.  Every factor is an
+// entry of the table itself.
+template <typename T>
+static std::vector<T> axis_twiddles(int n, int axis) {
+  std::vector<T> t = twiddles<T>(n);
+  t.resize(2 * (size_t)n * 3, (T)0);
+  std::vector<int> r = fft_schedule(n, axis, sizeof(T) == 4);
+  for (int order = 0; order < 2; ++order) {
+    size_t o = (size_t)(order + 1) * n;
+    int p = r.empty() ? 1 : r[0];
+    for (size_t s = 1; s < r.size(); ++s) {
+      for (int q = 1; q < r[s]; ++q)
+        for (int k = 0; k < p; ++k, ++o) {
+          const size_t m = (size_t)q * k * (n / (p * r[s]));
+          t[2 * o] = t[2 * m];
+          t[2 * o + 1] = t[2 * m + 1];
+        }
+      p *= r[s];
+    }
+    std::reverse(r.begin(), r.end());
+  }
+  return t;
+}
+
 template <typename T>
 static int upload_vec(void** dst, const std::vector<T>& v) {
   MHIT_CUDA_TRY(cudaMalloc(dst, v.size() * sizeof(T)));
@@ -687,12 +713,12 @@ static int init_impl(const mhit_params* p, mhit_ctx* c) {
   if (p->zsolve_tc && (rc = zsolve_tc_create(g, c->spec, &c->tcz))) return rc;
   if (ts == 4) {
     if ((rc = upload_vec(&c->twx, twiddles<float>(g.nx)))) return rc;
-    if ((rc = upload_vec(&c->twy, twiddles<float>(g.ny)))) return rc;
-    if ((rc = upload_vec(&c->twz, twiddles<float>(g.nz)))) return rc;
+    if ((rc = upload_vec(&c->twy, axis_twiddles<float>(g.ny, 1)))) return rc;
+    if ((rc = upload_vec(&c->twz, axis_twiddles<float>(g.nz, 2)))) return rc;
   } else {
     if ((rc = upload_vec(&c->twx, twiddles<double>(g.nx)))) return rc;
-    if ((rc = upload_vec(&c->twy, twiddles<double>(g.ny)))) return rc;
-    if ((rc = upload_vec(&c->twz, twiddles<double>(g.nz)))) return rc;
+    if ((rc = upload_vec(&c->twy, axis_twiddles<double>(g.ny, 1)))) return rc;
+    if ((rc = upload_vec(&c->twz, axis_twiddles<double>(g.nz, 2)))) return rc;
   }
   // k^2 per axis (multi/main.f90:234-240, 889), or the modified wavenumber.  The cells are cubes
   // of side dx = lx/nx, so an axis of nn cells is nn dx long: its wavenumber of index kk is
@@ -1476,7 +1502,8 @@ int mhit_energy_spectrum(mhit_ctx* c, double* E, int nbins) {
     if (!c->tw64[0]) {
       const int ns[3] = {g.nx, g.ny, g.nz};
       for (int q = 0; q < 3; ++q)
-        if ((rc = upload_vec(&c->tw64[q], twiddles<double>(ns[q])))) return rc;
+        if ((rc = upload_vec(&c->tw64[q], q == 0 ? twiddles<double>(ns[q]) : axis_twiddles<double>(ns[q], q))))
+        return rc;
     }
     spec = c->spec64;
     tx = c->tw64[0];
