@@ -40,6 +40,24 @@ template <int N, int B> __host__ __device__ constexpr int fft_threads() {
 
 template <int B> __device__ __forceinline__ int sw(int n, int b) { return n * B + (b ^ (n & (B - 1))); }
 
+// f(row, column) over B rows of LEN elements by the threads tid = 0..NT-1.  Rows of 64 and more go
+// row by row to the warps, so no thread divides its index by a length that is no power of two (the
+// half spectra's M + 1); short rows are dealt out element by element.
+template <int LEN, int B, int NT, typename F> __device__ __forceinline__ void for_rows(int tid, F f) {
+  if constexpr (LEN >= 64) {
+#pragma unroll
+    for (int b0 = 0; b0 < B; b0 += NT / 32) {
+      const int b = b0 + (tid >> 5);
+      if (B % (NT / 32) == 0 || b < B) {
+#pragma unroll 4
+        for (int c = tid & 31; c < LEN; c += 32) f(b, c);
+      }
+    }
+  } else {
+    for (int e = tid; e < LEN * B; e += NT) f(e / LEN, e % LEN);
+  }
+}
+
 // ---------------------------------------------------------------- register butterflies
 template <typename T, bool INV> __device__ __forceinline__ void dft2(Cx<T>* a) {
   Cx<T> t = a[0];

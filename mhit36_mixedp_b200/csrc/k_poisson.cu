@@ -236,11 +236,10 @@ k_div_fftx(const double* __restrict__ u, const double* __restrict__ v, const dou
   }
   __syncthreads();
   const int pitch = g.pitch;
-  for (int e = threadIdx.x; e < (M + 1) * B; e += NT) {
-    const int b = e / (M + 1), kx = e - b * (M + 1);
+  for_rows<M + 1, B, NT>(threadIdx.x, [&](int b, int kx) {
     const int line = line0 + b;
     if (line < nlines) spec[(size_t)line * pitch + kx] = s[sw<B>(kx, b)];
-  }
+  });
 }
 
 // ------------------------------------------------------------------ inverse x -> pressure
@@ -259,11 +258,10 @@ k_fftx_inv(const Cx<T>* __restrict__ spec, T* __restrict__ p, const Cx<T>* __res
   const int nlines = g.ny * g.nz;
   const int line0 = blockIdx.x * B;
   const int pitch = g.pitch;
-  for (int e = threadIdx.x; e < (M + 1) * B; e += NT) {
-    const int b = e / (M + 1), kx = e - b * (M + 1);
+  for_rows<M + 1, B, NT>(threadIdx.x, [&](int b, int kx) {
     const int line = min(line0 + b, nlines - 1);  // a tail tile repeats the last line
     __pipeline_memcpy_async(&s[sw<B>(kx, b)], &spec[(size_t)line * pitch + kx], sizeof(Cx<T>));
-  }
+  });
   __pipeline_commit();
   __pipeline_wait_prior(0);
   __syncthreads();

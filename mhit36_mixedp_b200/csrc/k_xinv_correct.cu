@@ -136,12 +136,11 @@ __global__ void __launch_bounds__(xc_nf<M>() + xc_ns<M>(), 1) k_xinv_correct(con
       kk = kk < 0 ? kk + nz : kk;
       const Cx<T>* src = spec + (size_t)kk * ny * pitch;
       Cx<T>* s = tiles + (i % XNB) * TL;
-      for (int e = tid; e < TL; e += NF) {
-        const int b = e / (M + 1), kx = e - b * (M + 1);
+      for_rows<M + 1, XL, NF>(tid, [&](int b, int kx) {
         int j = j0 - 1 + b;
         j = j < 0 ? j + ny : (j >= ny ? j - ny : j);
         __pipeline_memcpy_async(&s[sw<XL>(kx, b)], &src[(size_t)j * pitch + kx], sizeof(Cx<T>));
-      }
+      });
       if constexpr (INC) {
         // the same 8 lines of the predictor, 16-byte chunks (a line is nx floats, nx % 4 == 0)
         const float* qsrc = a.qold + (size_t)kk * ny * nx;
