@@ -98,7 +98,15 @@ __device__ __forceinline__ int pmod_int(int x, int n) {
 
 // One z column of MTX x MTY cells, tile (bx, by), chunk bz, of the box a, with the step's
 // alpha, beta (AB2 weights).
-template <bool PHI>
+//
+// CARRY: a thread carries its own column's u, v, w of planes k-1 and k, its chemical potential and its
+// last z force in registers instead of reading them from the rings again, 9 of 49 shared loads per
+// cell: the shared-memory pipe bounds the kernel (ncu: 79% of its wavefronts at 61% of the DRAM
+// bandwidth).  The same bits; 2.81 -> 2.75 ms at 512^3 and 386 -> 370 us at 256^3 on one box, 62 -> 58
+// us at 128^3.  Without the phase field nothing changes.  The batched kernel, whose arguments
+// take registers (they come from device memory), spills with it (ensemble of 32 boxes 4.55 -> 4.87
+// ms) and reads the rings.
+template <bool PHI, bool CARRY>
 __device__ __forceinline__ void mom_tile(const MomArgs& a, double alpha, double beta, int bx, int by, int bz,
                                          unsigned char* smraw) {
   MomSmem<PHI>& S = *reinterpret_cast<MomSmem<PHI>*>(smraw);
@@ -169,18 +177,35 @@ __device__ __forceinline__ void mom_tile(const MomArgs& a, double alpha, double 
   bool waits_ok = true;
 
   const double eps = g.eps, epsi = g.epsi, ddxi = g.ddxi, dxi = g.dxi;
+  const int tx = tid % MTX, ty = tid / MTX;
+  const int uq = (ty + 1) * UPX + (tx + 2);   // own cell in the u/v/w plane
+  const int pq = (ty + 2) * PPX + (tx + 2);   // own cell in the phi plane
+  const int cq = (ty + 1) * CPX + (tx + 1);   // own cell in the chempot plane
   // chemical potential (multi/main.f90:735) of plane m over the CPX x CPY region
+  double ca1 = 0.0, ca0 = 0.0, fzm = 0.0;  // CARRY: the own cell's at planes k+1 and k, its z force at k-1
   auto chempot_plane = [&](int m) {
     if constexpr (PHI) {
-      auto& P = reinterpret_cast<MomSmem<true>&>(S).phi;
-      const int pm = (m - k0 + 15) & 7, p0 = (m - k0 + 16) & 7, pp = (m - k0 + 17) & 7;
-      const int sc = (m - k0 + 16) & 3;
-      for (int e = tid; e < CPL; e += MNT) {
-        const int y = e / CPX, x = e - y * CPX;
-        const int q = (y + 1) * PPX + (x + 1);  // phi index of (i0-1+x, j0-1+y)
-        const double c = P[p0][q];
-        const double s = P[p0][q + 1] + P[p0][q - 1] + P[p0][q + PPX] + P[p0][q - PPX] + P[pp][q] + P[pm][q];
-        reinterpret_cast<MomSmem<true>&>(S).cp[sc][e] = c * (1.0 - c) * (1.0 - 2.0 * c) * epsi - eps * (s - 6.0 * c) * ddxi;
+      auto& SP = reinterpret_cast<MomSmem<true>&>(S);
+      const double* Pm = SP.phi[(m - k0 + 15) & 7];
+      const double* P0 = SP.phi[(m - k0 + 16) & 7];
+      const double* Pp = SP.phi[(m - k0 + 17) & 7];
+      double* C = SP.cp[(m - k0 + 16) & 3];
+      auto cell = [&](int q, int e) {
+        const double c = P0[q];
+        const double s = P0[q + 1] + P0[q - 1] + P0[q + PPX] + P0[q - PPX] + Pp[q] + Pm[q];
+        const double bulk = __dmul_rn(__dmul_rn(c, 1.0 - c), __fma_rn(-2.0, c, 1.0));
+        return C[e] = __fma_rn(bulk, epsi, -__dmul_rn(__dmul_rn(eps, __fma_rn(-6.0, c, s)), ddxi));
+      };
+      if constexpr (CARRY) {
+        // every thread its own cell, then row -1 (the first warp) and column -1 (the next threads)
+        ca1 = cell(pq, cq);
+        if (tid < MTX) cell(PPX + tid + 2, tid + 1);
+        else if (tid < MTX + CPY) cell((tid - MTX + 1) * PPX + 1, (tid - MTX) * CPX);
+      } else {
+        for (int e = tid; e < CPL; e += MNT) {
+          const int y = e / CPX, x = e - y * CPX;
+          cell((y + 1) * PPX + (x + 1), e);
+        }
       }
     }
   };
@@ -221,7 +246,6 @@ __device__ __forceinline__ void mom_tile(const MomArgs& a, double alpha, double 
     __pipeline_commit();
   }
 
-  const int tx = tid % MTX, ty = tid / MTX;
   const int i = i0 + tx, j = j0 + ty;
   const bool own = i < nx && j < ny;
   const double* t = a.tabs;
@@ -233,10 +257,9 @@ __device__ __forceinline__ void mom_tile(const MomArgs& a, double alpha, double 
   const double c_vis = g.mu * ddxi * g.rhoi;           // mu lap(u) / rho
   const double c_st = 6.0 * g.sigma * 0.25 * dxi * g.rhoi;  // face average of the force / rho
   const double dta = g.dt * alpha, dtb = g.dt * beta;
-  const int uq = (ty + 1) * UPX + (tx + 2);   // own cell in the u/v/w plane
-  const int pq = (ty + 2) * PPX + (tx + 2);   // own cell in the phi plane
-  const int cq = (ty + 1) * CPX + (tx + 1);   // own cell in the chempot plane
 
+  // own u, v, w of planes k and k-1 (carried from plane to plane: CARRY)
+  double u0 = 0.0, v0 = 0.0, w0 = 0.0, uzm = 0.0, vzm = 0.0, wzm = 0.0;
   // four planes per unrolled body: 2.86 ms at 512^3 against 2.91 not unrolled and 2.93 unrolled
   // twice; the same bits
 #pragma unroll 4
@@ -272,19 +295,28 @@ __device__ __forceinline__ void mom_tile(const MomArgs& a, double alpha, double 
       }
     }
     if (!tma) __pipeline_commit();
+    ca0 = ca1;
     if (k + 1 < k1) chempot_plane(k + 1);
+    if constexpr (PHI && CARRY) {
+      // the z force of the plane below the chunk, the first output plane's -z neighbour
+      if (k == k0 - 1) {
+        auto& P = reinterpret_cast<MomSmem<true>&>(S).phi;
+        fzm = __dmul_rn(ca0, P[0][pq] - P[6][pq]);
+      }
+    }
     if (out) {
       const int sm = (k - k0 + 15) & 3, s0 = (k - k0 + 16) & 3, sp = (k - k0 + 17) & 3;
       const double* U0 = S.u[s0];
       const double* V0 = S.v[s0];
       const double* W0 = S.w[s0];
-      const double u0 = U0[uq] - mu_, v0 = V0[uq] - mv_, w0 = W0[uq] - mw_;
+      if (!CARRY || k == k0) u0 = U0[uq] - mu_, v0 = V0[uq] - mv_, w0 = W0[uq] - mw_;
       const double uxp = U0[uq + 1] - mu_, uxm = U0[uq - 1] - mu_, uyp = U0[uq + UPX] - mu_, uym = U0[uq - UPX] - mu_;
-      const double uzp = S.u[sp][uq] - mu_, uzm = S.u[sm][uq] - mu_;
+      const double uzp = S.u[sp][uq] - mu_;
+      if (!CARRY || k == k0) uzm = S.u[sm][uq] - mu_, vzm = S.v[sm][uq] - mv_, wzm = S.w[sm][uq] - mw_;
       const double vxp = V0[uq + 1] - mv_, vxm = V0[uq - 1] - mv_, vyp = V0[uq + UPX] - mv_, vym = V0[uq - UPX] - mv_;
-      const double vzp = S.v[sp][uq] - mv_, vzm = S.v[sm][uq] - mv_;
+      const double vzp = S.v[sp][uq] - mv_;
       const double wxp = W0[uq + 1] - mw_, wxm = W0[uq - 1] - mw_, wyp = W0[uq + UPX] - mw_, wym = W0[uq - UPX] - mw_;
-      const double wzp = S.w[sp][uq] - mw_, wzm = S.w[sm][uq] - mw_;
+      const double wzp = S.w[sp][uq] - mw_;
       const double v_imjp = V0[uq + UPX - 1] - mv_, w_imkp = S.w[sp][uq - 1] - mw_, u_ipjm = U0[uq - UPX + 1] - mu_;
       const double w_jmkp = S.w[sp][uq - UPX] - mw_, u_ipkm = S.u[sm][uq + 1] - mu_, v_jpkm = S.v[sm][uq + UPX] - mv_;
       // multi/main.f90:672-694: the fluxes h = a^2 - b^2 and h = a c - b d as one product and
@@ -317,14 +349,17 @@ __device__ __forceinline__ void mom_tile(const MomArgs& a, double alpha, double 
         // 6 sigma mu_c grad(phi) / rho averaged to the face, the central differences taken as
         // (phi+ - phi-) dxi / 2
         auto& SP = reinterpret_cast<MomSmem<true>&>(S);
-        const int pmm = (k - k0 + 14) & 7, pm = (k - k0 + 15) & 7, p0 = (k - k0 + 16) & 7, pp = (k - k0 + 17) & 7;
-        const int c0s = (k - k0 + 16) & 3, cms = (k - k0 + 15) & 3;
+        const int pm = (k - k0 + 15) & 7, p0 = (k - k0 + 16) & 7, pp = (k - k0 + 17) & 7;
+        const int c0s = (k - k0 + 16) & 3;
+        const double dz = SP.phi[pp][pq] - SP.phi[pm][pq];
         const double* P0 = SP.phi[p0];
         const double pc = P0[pq];
-        const double c0 = SP.cp[c0s][cq];
+        const double c0 = CARRY ? ca0 : SP.cp[c0s][cq];
         const double fx = __fma_rn(c0, P0[pq + 1] - P0[pq - 1], SP.cp[c0s][cq - 1] * (pc - P0[pq - 2]));
         const double fy = __fma_rn(c0, P0[pq + PPX] - P0[pq - PPX], SP.cp[c0s][cq - CPX] * (pc - P0[pq - 2 * PPX]));
-        const double fz = __fma_rn(c0, SP.phi[pp][pq] - SP.phi[pm][pq], SP.cp[cms][cq] * (pc - SP.phi[pmm][pq]));
+        if (!CARRY) fzm = SP.cp[(k - k0 + 15) & 3][cq] * (pc - SP.phi[(k - k0 + 14) & 7][pq]);
+        const double fz = __fma_rn(c0, dz, fzm);
+        if (CARRY) fzm = __dmul_rn(c0, dz);
         ru = __fma_rn(c_st, fx, ru);
         rv = __fma_rn(c_st, fy, rv);
         rw = __fma_rn(c_st, fz, rw);
@@ -336,6 +371,7 @@ __device__ __forceinline__ void mom_tile(const MomArgs& a, double alpha, double 
       a.ru[c] = ru;
       a.rv[c] = rv;
       a.rw[c] = rw;
+      if (CARRY) uzm = u0, vzm = v0, wzm = w0, u0 = uzp, v0 = vzp, w0 = wzp;
     }
   }
   __pipeline_wait_prior(0);
@@ -347,7 +383,7 @@ __device__ __forceinline__ void mom_tile(const MomArgs& a, double alpha, double 
 template <bool PHI>
 __global__ void __launch_bounds__(MNT, 3) k_mom(const __grid_constant__ MomArgs a) {
   extern __shared__ __align__(128) unsigned char smraw[];
-  mom_tile<PHI>(a, a.alpha, a.beta, blockIdx.x, blockIdx.y, blockIdx.z, smraw);
+  mom_tile<PHI, true>(a, a.alpha, a.beta, blockIdx.x, blockIdx.y, blockIdx.z, smraw);
 }
 
 // The momentum step of many boxes in one launch: persistent blocks (three per SM) take work items
@@ -364,7 +400,7 @@ __global__ void __launch_bounds__(MNT, 3) k_mom_batch(const __grid_constant__ Ba
     __syncthreads();  // every thread has the item before thread 0 takes the next one
     if (it >= b.nitems) break;
     const int4 w = b.items[it];
-    mom_tile<PHI>(b.args[w.x], b.alpha, b.beta, w.y, w.z, w.w, smraw);
+    mom_tile<PHI, false>(b.args[w.x], b.alpha, b.beta, w.y, w.z, w.w, smraw);
     __syncthreads();  // the rings are reused by the next item
   }
 }
