@@ -100,9 +100,12 @@ struct mhit_ctx {
   int mom_tma = 1;                        // k_mom fills its interior rings by TMA (test hook: 0)
   int graph_kernels = 0;                  // kernel nodes in a captured step graph
   // 1: the inverse x transform runs fused with the projection (k_xinv_correct); 0: k_fftx_inv +
-  // k_correct; -1 (the default): fused where that is the faster, nx = 512 (measured at 512^3:
-  // FP64 pass pair 1.63 against 1.77 ms; at 1024^3, where k_correct streams at 96% of the copy
-  // peak, and on the small boxes of the ensemble the separate passes are faster).  The fused
+  // k_correct; -1 (the default): fused where that is the faster.  Step times of the two without the
+  // phase field, separate / fused: nx = 512 from 8192 x lines on (512x128x64 FP64 232 / 227 us, FP32
+  // 194 / 190, incremental 216 / 207; 512x64x64 117 / 135, 105 / 119, 120 / 131); nx = 256 in FP64 from
+  // 65536 lines on (256^3 849 / 826 us, 256x1024x64 888 / 851; 256x128x128 240 / 244; FP32 always
+  // slower, 256^3 689 / 713).  At 192 points and less, and at 1024^3, where k_correct streams at 96%
+  // of the copy peak, the separate passes are faster.  The fused
   // pass leaves the pressure in the spectrum only: after such a step p_lazy is set, and whatever
   // reads the pressure or reuses the spectrum first materialises it (materialise_pressure).
   int fuse_xc = -1;
@@ -118,7 +121,10 @@ static bool incremental(const mhit_ctx* c) { return c->prm.poisson == MHIT_POISS
 // whose projection reads the sum of two pressures)
 static bool fused_xc(const mhit_ctx* c) {
   if (refined(c)) return false;
-  return c->fuse_xc >= 0 ? c->fuse_xc != 0 : c->g.nx == 512;
+  if (c->fuse_xc >= 0) return c->fuse_xc != 0;
+  const long long lines = (long long)c->g.ny * c->g.nz;
+  if (c->g.nx == 512) return lines >= 8192;
+  return c->g.nx == 256 && c->prm.poisson == MHIT_POISSON_FP64 && lines >= 65536;
 }
 
 static int check_ctx(mhit_ctx* c) {
