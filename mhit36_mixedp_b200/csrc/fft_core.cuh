@@ -188,19 +188,24 @@ template <typename T, bool INV, int R> __device__ __forceinline__ void dftR(Cx<T
 // barrier (id, count) when only some warps of the block transform (warp-specialised kernels).
 struct SyncBlock {
   __device__ __forceinline__ static void sync() { __syncthreads(); }
+  __device__ __forceinline__ static int tid() { return threadIdx.x; }
 };
-template <int ID, int COUNT> struct SyncNamed {
-  __device__ __forceinline__ static void sync() { asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(COUNT) : "memory"); }
+// the groups of COUNT threads 0.., COUNT.., each on named barrier 1 + its number
+template <int COUNT> struct SyncGroup {
+  __device__ __forceinline__ static void sync() {
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + (int)threadIdx.x / COUNT), "n"(COUNT) : "memory");
+  }
+  __device__ __forceinline__ static int tid() { return threadIdx.x % COUNT; }
 };
 
 // ---------------------------------------------------------------- one Stockham stage
-// tw: table of exp(-2 pi i m / L) for m in [0, L); twstride = L / N.  Threads 0..NT-1 take part.
+// tw: table of exp(-2 pi i m / L) for m in [0, L); twstride = L / N.  Threads 0..NT-1 (of SY) take part.
 template <typename T, int N, int B, int NT, int R, bool INV, typename SY = SyncBlock>
 __device__ __forceinline__ void stockham_stage(Cx<T>* s, const Cx<T>* __restrict__ tw, int twstride, int p) {
   constexpr int NB = N / R * B;
   constexpr int BPT = (NB + NT - 1) / NT;
   Cx<T> a[BPT][R];
-  const int tid = threadIdx.x;
+  const int tid = SY::tid();
 #pragma unroll
   for (int m = 0; m < BPT; ++m) {
     const int q = tid + m * NT;
@@ -264,9 +269,9 @@ __device__ __forceinline__ void fft_tile(Cx<T>* s, const Cx<T>* __restrict__ tw,
 // packed half-length sequence Z[k] = (X[k] + X*[M-k]) + i W^-k (X[k] - X*[M-k]), W = exp(-2 pi
 // i/(2M)), whose inverse transform gives the real line as (even + i odd) pairs; the imaginary
 // parts of X[0] and X[M] are ignored.  Caller synchronises before (tile loaded) and after.
-template <typename T, int M, int B, int NT>
+template <typename T, int M, int B, int NT, typename SY = SyncBlock>
 __device__ __forceinline__ void c2r_untangle(Cx<T>* s, const Cx<T>* __restrict__ twx) {
-  for (int e = threadIdx.x; e < (M / 2 + 1) * B; e += NT) {
+  for (int e = SY::tid(); e < (M / 2 + 1) * B; e += NT) {
     const int kk = e / B, b = e - kk * B;
     if (kk == 0) {
       const T a = s[sw<B>(0, b)].x, c = s[sw<B>(M, b)].x;

@@ -5,23 +5,25 @@
 // pressure's -x, -y and -z neighbours of each cell).  Here a block owns XO = 7 consecutive y
 // lines of a chunk of z planes and marches up z.  Per plane the block
 //   1. fetches the plane's 8 half-spectrum rows (its 7 lines and the line below them, j0 - 1,
-//      the -y neighbour of its first line) with cp.async, two planes ahead, into a ring of three
-//      tile buffers in shared memory;
+//      the -y neighbour of its first line) with cp.async into a ring of four tile buffers in
+//      shared memory (three at nx = 1024);
 //   2. C2R-transforms the 8 rows in place (the untangle and the Stockham stages of k_fftx_inv, so
 //      the on-demand transform of the same spectrum gives the same doubles);
 //   3. projects its 7 lines (u -= dt/rho (p - p(i-1)) dxi, and v, w along y, z: :953-955) with
-//      p(i-1) and p(j-1) from the tile and p(k-1) carried by each thread for its own x pairs from
-//      the plane below (the loop starts one plane below the chunk for them), and accumulates the
-//      per-block sums and maxima of k_correct.
-// The warps are specialised so the two kinds of work overlap: the transform warps (steps 1-2,
-// synchronising among themselves on named barrier 1) transform plane i while the stream warps
-// (step 3: the u, v, w traffic) project plane i - 1.  At nx = 512 each stream thread stages its
-// u, v, w pairs of the next plane in shared memory by cp.async as it finishes each pair of the
-// current one, so a whole plane's loads are in flight without holding registers.  A tile buffer
-// passes between them by named barriers: "ready" (2 + buffer: transform warps arrive, stream
-// warps wait) and "free" (5 + buffer: stream warps arrive, transform warps wait before fetching
-// plane i + 2 into the buffer of plane i - 1).  Hardware barriers, no spin loops; every arrival
-// has its matching wait, and a barrier's next phase starts only after its last one completed.
+//      p(i-1) and p(j-1) from the tile and p(k-1) from the tile of the plane below (the loop starts
+//      one plane below the chunk for it; at nx = 1024 each thread carries it), and accumulates
+//      the per-block sums and maxima of k_correct.
+// The warps are specialised so the two kinds of work overlap: two groups of transform warps (steps
+// 1-2; one group for the even planes, one for the odd, each synchronising on a named barrier of
+// its own; a single group at nx = 1024) run ahead of the stream warps (step 3: the u, v, w
+// traffic).  Up to nx = 512 each stream thread stages its u, v, w pairs of the next plane in shared
+// memory by cp.async as it finishes each pair of the current one, so a whole plane's loads are in
+// flight without holding registers.  A tile buffer passes between them by named barriers, one of
+// each kind per buffer: "ready" (a transform group arrives, the stream warps wait) and "free" (the
+// stream warps arrive once they have finished the plane above, which reads the buffer last; the
+// group that fetches the plane four further up into it waits).  Hardware barriers, no spin loops;
+// every arrival has its matching wait, and a barrier's next phase starts only after its last one
+// completed.
 //
 // The pressure never goes to HBM: the library transforms it from the spectrum, which stays intact
 // until the next step's x pass, when something reads it.  Per cell this moves the spectrum once
@@ -45,7 +47,6 @@ namespace mhit {
 constexpr int XL = 8;       // lines transformed per plane (a power of two: the tile swizzle)
 constexpr int XO = XL - 1;  // lines projected per plane: tile line 0 is the -y halo
 constexpr int XZC_MIN = 8;  // fewest z planes per block of the default chunking
-constexpr int XNB = 3;      // tile buffers: loading, transforming, being projected
 
 // transform threads: one butterfly of the schedule's largest radix each (at most 256: larger tiles
 // loop), at least 64
@@ -60,25 +61,36 @@ template <int M> __host__ __device__ constexpr int xc_nf() {
 // stream threads: 7 x pairs of the 7 lines each at nx = 512, 14 at nx = 1024
 template <int M> __host__ __device__ constexpr int xc_ns() { return M >= 256 ? 256 : 128; }
 template <int M> __host__ __device__ constexpr int xc_ppt() { return (XO * M + xc_ns<M>() - 1) / xc_ns<M>(); }
-template <typename T, int M> __host__ __device__ constexpr size_t xc_spec_bytes() {
-  return (size_t)XNB * (M + 1) * XL * sizeof(Cx<T>);
+// one tile buffer: the spectrum rows and, in the incremental solve, beside them the 8 lines of the
+// FP32 predictor (row-major)
+template <typename T, int M, bool INC> __host__ __device__ constexpr size_t xc_buffer_bytes() {
+  return (size_t)(M + 1) * XL * sizeof(Cx<T>) + (INC ? (size_t)XL * 2 * M * sizeof(float) : 0);
 }
-// incremental solve: beside each spectrum tile, the 8 lines of the FP32 predictor (row-major)
-template <typename T, int M, bool INC> __host__ __device__ constexpr size_t xc_tile_bytes() {
-  return xc_spec_bytes<T, M>() + (INC ? (size_t)XNB * XL * 2 * M * sizeof(float) : 0);
+// Two groups of transform warps, one for the even planes and one for the odd ones, over four tile
+// buffers (the stream warps take the -z neighbour's pressure from the buffer of the plane below, which
+// they hold one plane longer), up to nx = 512 (at 1024 four buffers do not fit in FP64).  One group's
+// transform of a plane (load wait, untangle, two radix-16 stages with barriers) takes longer in FP64
+// than the plane's u, v, w traffic, and with one group the stream warps waited for it: at 512^3 1715 ->
+// 1428 us in FP64, 1513 -> 1400 us in the incremental solve, 1220 -> 1183 us in FP32 (the copy peak
+// allows 1150, 1230 and 1070).
+// Otherwise one group over three buffers, the pressure carried to the next plane by the stream
+// threads.
+template <typename T, int M, bool INC> __host__ __device__ constexpr int xc_ng() {
+  return M <= 256 ? 2 : 1;
 }
-// The pressure each stream thread carries to the next plane (the -z neighbour) lives in shared
-// memory where it fits beside the tiles (in registers it would crowd out the loads), else in
-// registers (FP64 at nx = 1024).
-template <typename T, int M, bool INC> __host__ __device__ constexpr bool xc_pz_shared() {
-  return xc_tile_bytes<T, M, INC>() + (size_t)xc_ns<M>() * xc_ppt<M>() * 16 <= 227 * 1024;
+template <typename T, int M, bool INC> __host__ __device__ constexpr int xc_nb() { return xc_ng<T, M, INC>() + 2; }
+template <typename T, int M, bool INC> __host__ __device__ constexpr int xc_nt() {
+  return xc_ng<T, M, INC>() * xc_nf<M>() + xc_ns<M>();
+}
+template <typename T, int M, bool INC> __host__ __device__ constexpr size_t xc_spec_bytes() {
+  return (size_t)xc_nb<T, M, INC>() * (M + 1) * XL * sizeof(Cx<T>);
 }
 template <typename T, int M, bool INC> __host__ __device__ constexpr size_t xc_smem() {
-  return xc_tile_bytes<T, M, INC>() + (xc_pz_shared<T, M, INC>() ? (size_t)xc_ns<M>() * xc_ppt<M>() * 16 : 0);
+  return xc_nb<T, M, INC>() * xc_buffer_bytes<T, M, INC>();
 }
 // where the loads go through registers: x pairs a stream thread loads before computing any of them
 template <typename T, int M, bool INC> __host__ __device__ constexpr int xc_pb() {
-  return xc_pz_shared<T, M, INC>() ? 7 : 2;
+  return xc_ng<T, M, INC>() == 2 ? 7 : 2;
 }
 // Where it fits as well (nx = 512), each stream thread stages its u, v, w pairs of the NEXT plane
 // in shared memory with cp.async, pair by pair as it finishes the current plane's pair (one
@@ -88,7 +100,7 @@ template <typename T, int M, bool INC> __host__ __device__ constexpr size_t xc_u
   return (size_t)3 * xc_ns<M>() * xc_ppt<M>() * 16;
 }
 template <typename T, int M, bool INC> __host__ __device__ constexpr bool xc_uvw_shared() {
-  return xc_pz_shared<T, M, INC>() && xc_smem<T, M, INC>() + xc_uvw_bytes<T, M, INC>() <= 227 * 1024;
+  return xc_ng<T, M, INC>() == 2 && xc_smem<T, M, INC>() + xc_uvw_bytes<T, M, INC>() <= 227 * 1024;
 }
 template <typename T, int M, bool INC> __host__ __device__ constexpr size_t xc_smem_all() {
   return xc_smem<T, M, INC>() + (xc_uvw_shared<T, M, INC>() ? xc_uvw_bytes<T, M, INC>() : 0);
@@ -102,19 +114,21 @@ __device__ __forceinline__ void bar_arrive(int id, int count) {
 }
 
 template <typename T, int M, bool INC>
-__global__ void __launch_bounds__(xc_nf<M>() + xc_ns<M>(), 1) k_xinv_correct(const XcArgs a) {
-  constexpr int NF = xc_nf<M>(), NS = xc_ns<M>(), NT = NF + NS;
+__global__ void __launch_bounds__(xc_nt<T, M, INC>(), 1) k_xinv_correct(const XcArgs a) {
+  constexpr int NF = xc_nf<M>(), NS = xc_ns<M>(), NT = xc_nt<T, M, INC>();
+  constexpr int NG = xc_ng<T, M, INC>(), XNB = xc_nb<T, M, INC>();
+  constexpr int PAIR = NF + NS;            // threads of a hand-over: one transform group, the stream warps
+  constexpr int READY = 1 + NG, FREE = READY + XNB;  // named barriers: 1.. the groups', then per buffer
   constexpr int TL = (M + 1) * XL;         // elements of one tile buffer
   constexpr int NP = XO * M;               // x pairs projected per plane
   constexpr int PPT = xc_ppt<M>();         // ... per stream thread
   constexpr int XPB = xc_pb<T, M, INC>();
-  constexpr bool PZS = xc_pz_shared<T, M, INC>();
   constexpr bool UVS = xc_uvw_shared<T, M, INC>();
   constexpr int nx = 2 * M;
   constexpr int QL = XL * nx;              // floats of one predictor tile
   extern __shared__ __align__(16) unsigned char smraw[];
   Cx<T>* tiles = reinterpret_cast<Cx<T>*>(smraw);
-  float* qtiles = reinterpret_cast<float*>(smraw + xc_spec_bytes<T, M>());
+  float* qtiles = reinterpret_cast<float*>(smraw + xc_spec_bytes<T, M, INC>());
   const Geo& g = a.g;
   const int ny = g.ny, nz = g.nz;
   const int j0 = blockIdx.x * XO;
@@ -124,8 +138,10 @@ __global__ void __launch_bounds__(xc_nf<M>() + xc_ns<M>(), 1) k_xinv_correct(con
   double su = 0.0, sv = 0.0, sw_ = 0.0;
   double mu = -INFINITY, mv = -INFINITY, mw = -INFINITY;
 
-  if (tid < NF) {
+  if (tid < NG * NF) {
     // ---------------------------------------------------------- transform warps
+    using SY = SyncGroup<NF>;
+    const int gt = SY::tid(), grp = tid / NF;
     const Cx<T>* __restrict__ spec = static_cast<const Cx<T>*>(a.spec);
     const Cx<T>* __restrict__ twx = static_cast<const Cx<T>*>(a.twx);
     const int pitch = g.pitch;
@@ -136,7 +152,7 @@ __global__ void __launch_bounds__(xc_nf<M>() + xc_ns<M>(), 1) k_xinv_correct(con
       kk = kk < 0 ? kk + nz : kk;
       const Cx<T>* src = spec + (size_t)kk * ny * pitch;
       Cx<T>* s = tiles + (i % XNB) * TL;
-      for_rows<M + 1, XL, NF>(tid, [&](int b, int kx) {
+      for_rows<M + 1, XL, NF>(gt, [&](int b, int kx) {
         int j = j0 - 1 + b;
         j = j < 0 ? j + ny : (j >= ny ? j - ny : j);
         __pipeline_memcpy_async(&s[sw<XL>(kx, b)], &src[(size_t)j * pitch + kx], sizeof(Cx<T>));
@@ -145,7 +161,7 @@ __global__ void __launch_bounds__(xc_nf<M>() + xc_ns<M>(), 1) k_xinv_correct(con
         // the same 8 lines of the predictor, 16-byte chunks (a line is nx floats, nx % 4 == 0)
         const float* qsrc = a.qold + (size_t)kk * ny * nx;
         float* qs = qtiles + (i % XNB) * QL;
-        for (int e = tid; e < QL / 4; e += NF) {
+        for (int e = gt; e < QL / 4; e += NF) {
           const int b = e / (nx / 4), c4 = e - b * (nx / 4);
           int j = j0 - 1 + b;
           j = j < 0 ? j + ny : (j >= ny ? j - ny : j);
@@ -154,43 +170,51 @@ __global__ void __launch_bounds__(xc_nf<M>() + xc_ns<M>(), 1) k_xinv_correct(con
       }
       __pipeline_commit();
     };
-    fetch(0);
-    if (nplanes > 1) fetch(1);
-    for (int i = 0; i < nplanes; ++i) {
-      Cx<T>* s = tiles + (i % XNB) * TL;
-      if (i + 1 < nplanes) __pipeline_wait_prior(1);  // plane i's rows (plane i+1's may still fly)
-      else __pipeline_wait_prior(0);
-      bar_sync(1, NF);
-      c2r_untangle<T, M, XL, NF>(s, twx);
-      bar_sync(1, NF);
-      fft_tile<T, M, XL, NF, true, Radix<M>, SyncNamed<1, NF>>(s, twx, 2);
-      bar_arrive(2 + i % XNB, NT);  // plane i's pressure is in its buffer
-      if (i + 2 < nplanes) {
-        // the buffer of plane i + 2 held plane i - 1: wait until the stream warps are done with it
-        if (i >= 1) bar_sync(5 + (i - 1) % XNB, NT);
-        fetch(i + 2);
+    if constexpr (NG == 2) {
+      // plane i's buffer held plane i - 4, which the stream warps read until they finish plane i - 3
+      if (grp < nplanes) fetch(grp);
+      for (int i = grp; i < nplanes; i += 2) {
+        Cx<T>* s = tiles + (i % XNB) * TL;
+        __pipeline_wait_prior(0);
+        SY::sync();
+        c2r_untangle<T, M, XL, NF, SY>(s, twx);
+        SY::sync();
+        fft_tile<T, M, XL, NF, true, Radix<M>, SY>(s, twx, 2);
+        bar_arrive(READY + i % XNB, PAIR);  // plane i's pressure is in its buffer
+        if (i + 2 < nplanes) {
+          if (i >= 2) bar_sync(FREE + (i - 2) % XNB, PAIR);
+          fetch(i + 2);
+        }
+      }
+    } else {
+      fetch(0);
+      if (nplanes > 1) fetch(1);
+      for (int i = 0; i < nplanes; ++i) {
+        Cx<T>* s = tiles + (i % XNB) * TL;
+        if (i + 1 < nplanes) __pipeline_wait_prior(1);  // plane i's rows (plane i+1's may still fly)
+        else __pipeline_wait_prior(0);
+        SY::sync();
+        c2r_untangle<T, M, XL, NF, SY>(s, twx);
+        SY::sync();
+        fft_tile<T, M, XL, NF, true, Radix<M>, SY>(s, twx, 2);
+        bar_arrive(READY + i % XNB, PAIR);  // plane i's pressure is in its buffer
+        if (i + 2 < nplanes) {
+          // the buffer of plane i + 2 held plane i - 1: wait until the stream warps are done with it
+          if (i >= 1) bar_sync(FREE + (i - 1) % XNB, PAIR);
+          fetch(i + 2);
+        }
       }
     }
   } else {
     // ---------------------------------------------------------- stream warps
-    const int st = tid - NF;
+    const int st = tid - NG * NF;
     const size_t plane = (size_t)nx * ny;
     double* __restrict__ U = a.u;
     double* __restrict__ V = a.v;
     double* __restrict__ W = a.w;
     const double cc = g.dt / g.rho, dxi = g.dxi;
-    // pressure of the thread's x pairs at the plane below: [pair][stream thread] in shared memory
-    // after the tiles (each thread its own 16-byte slots: conflict-free), or in registers
-    double2* pzs = reinterpret_cast<double2*>(smraw + xc_tile_bytes<T, M, INC>()) + st;
-    double2 pzr[PZS ? 1 : PPT] = {};
-    auto pz_get = [&](int m) -> double2 {
-      if constexpr (PZS) return pzs[m * NS];
-      else return pzr[m];
-    };
-    auto pz_set = [&](int m, double2 v) {
-      if constexpr (PZS) pzs[m * NS] = v;
-      else pzr[m] = v;
-    };
+    // NG == 1: pressure of the thread's x pairs at the plane below
+    double2 pzr[NG == 1 ? PPT : 1] = {};
     // staged u, v, w of pair m, field f: uvs[(f * PPT + m) * NS] (each thread its own slots)
     double2* uvs = reinterpret_cast<double2*>(smraw + xc_smem<T, M, INC>()) + st;
     // pair m of plane index ip into its slots, as one commit group (empty for pairs without a cell,
@@ -214,9 +238,26 @@ __global__ void __launch_bounds__(xc_nf<M>() + xc_ns<M>(), 1) k_xinv_correct(con
     for (int i = 0; i < nplanes; ++i) {
       const Cx<T>* s = tiles + (i % XNB) * TL;
       const float* qs = qtiles + (i % XNB) * QL;
+      // the plane below's buffer (NG == 2; not read for i = 0)
+      const Cx<T>* sb = tiles + ((i + XNB - 1) % XNB) * TL;
+      const float* qb = qtiles + ((i + XNB - 1) % XNB) * QL;
+      // pressure of pair m (tile position n, line l + 1) at the plane below
+      auto below = [&](int m, int n, int l) -> double2 {
+        if constexpr (NG == 2) {
+          const Cx<T> z = sb[sw<XL>(n, l + 1)];
+          if constexpr (INC) {
+            const float2 q = *reinterpret_cast<const float2*>(qb + (l + 1) * nx + 2 * n);
+            return make_double2((double)q.x + (double)z.x, (double)q.y + (double)z.y);
+          } else {
+            return make_double2((double)z.x, (double)z.y);
+          }
+        } else {
+          return pzr[m];
+        }
+      };
       const int k = k0 - 1 + i;
       const int kk = k < 0 ? k + nz : k;
-      bar_sync(2 + i % XNB, NT);  // plane i's pressure (and predictor rows) are ready
+      bar_sync(READY + i % XNB, PAIR);  // plane i's pressure (and predictor rows) are ready
       if constexpr (UVS) {
 #pragma unroll
         for (int m = 0; m < PPT; ++m) {
@@ -255,7 +296,7 @@ __global__ void __launch_bounds__(xc_nf<M>() + xc_ns<M>(), 1) k_xinv_correct(con
               // multi/main.f90:953-955, the expressions of k_correct
               const double u0 = uo.x - cc * (p0 - pxm) * dxi, u1 = uo.y - cc * (p1 - p0) * dxi;
               const double v0 = vo.x - cc * (p0 - py0) * dxi, v1 = vo.y - cc * (p1 - py1) * dxi;
-              const double2 pk = pz_get(m);
+              const double2 pk = below(m, n, l);
               const double w0 = wo.x - cc * (p0 - pk.x) * dxi, w1 = wo.y - cc * (p1 - pk.y) * dxi;
               *reinterpret_cast<double2*>(U + o) = make_double2(u0, u1);
               *reinterpret_cast<double2*>(V + o) = make_double2(v0, v1);
@@ -268,7 +309,7 @@ __global__ void __launch_bounds__(xc_nf<M>() + xc_ns<M>(), 1) k_xinv_correct(con
               mv = fmax(mv, fmax(v0, v1));
               mw = fmax(mw, fmax(w0, w1));
             }
-            pz_set(m, make_double2(p0, p1));
+            if constexpr (NG == 1) pzr[m] = make_double2(p0, p1);
           }
           // the slots are free (their values consumed above): the next plane's pair goes in
           stage_pair(i + 1, m);
@@ -328,7 +369,7 @@ __global__ void __launch_bounds__(xc_nf<M>() + xc_ns<M>(), 1) k_xinv_correct(con
                 // multi/main.f90:953-955, the expressions of k_correct
                 const double u0 = uo[mb].x - cc * (p0 - pxm) * dxi, u1 = uo[mb].y - cc * (p1 - p0) * dxi;
                 const double v0 = vo[mb].x - cc * (p0 - py0) * dxi, v1 = vo[mb].y - cc * (p1 - py1) * dxi;
-                const double2 pk = pz_get(m);
+                const double2 pk = below(m, n, l);
                 const double w0 = wo[mb].x - cc * (p0 - pk.x) * dxi, w1 = wo[mb].y - cc * (p1 - pk.y) * dxi;
                 *reinterpret_cast<double2*>(U + o) = make_double2(u0, u1);
                 *reinterpret_cast<double2*>(V + o) = make_double2(v0, v1);
@@ -341,13 +382,20 @@ __global__ void __launch_bounds__(xc_nf<M>() + xc_ns<M>(), 1) k_xinv_correct(con
                 mv = fmax(mv, fmax(v0, v1));
                 mw = fmax(mw, fmax(w0, w1));
               }
-              pz_set(m, make_double2(p0, p1));
+              if constexpr (NG == 1) pzr[m] = make_double2(p0, p1);
             }
           }
         }
       }
-      // the transform warps wait for this buffer only if they fetch plane i + 3 into it
-      if (i + 3 < nplanes) bar_arrive(5 + i % XNB, NT);
+      // the transform warps wait for a buffer only if they fetch another plane into it: plane i + 3
+      // into that of plane i - 1 (NG == 2: read for the last time here) or of plane i
+      if (i + 3 < nplanes) {
+        if constexpr (NG == 2) {
+          if (i >= 1) bar_arrive(FREE + (i - 1) % XNB, PAIR);
+        } else {
+          bar_arrive(FREE + i % XNB, PAIR);
+        }
+      }
     }
     if constexpr (UVS) __pipeline_wait_prior(0);  // no copy into the block's shared memory outlives it
   }
@@ -399,7 +447,6 @@ int xc_blocks(const Geo& g, int zc) {
 
 template <typename T, int M>
 static cudaError_t launch_xc_m(const XcArgs& a, cudaStream_t st) {
-  constexpr int NT = xc_nf<M>() + xc_ns<M>();
   // the incremental solve is an FP32 mode: its variant exists for float tiles only
   constexpr bool HAS_INC = sizeof(T) == 4;
   static_assert(xc_smem_all<T, M, false>() <= 227 * 1024 && (!HAS_INC || xc_smem_all<T, M, HAS_INC>() <= 227 * 1024),
@@ -413,7 +460,8 @@ static cudaError_t launch_xc_m(const XcArgs& a, cudaStream_t st) {
   XcArgs b = a;
   b.zc = xc_chunk(a.g, a.zc);
   const dim3 grid = xc_grid(a.g, a.zc);
-  kern<<<grid, NT, smem, st>>>(b);
+  const int nt = a.qold ? xc_nt<T, M, HAS_INC>() : xc_nt<T, M, false>();
+  kern<<<grid, nt, smem, st>>>(b);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   return launch_finalize(a.partials, (int)(grid.x * grid.y), a.g, a.sc, a.sc_host, st);

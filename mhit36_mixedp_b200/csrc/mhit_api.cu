@@ -100,12 +100,14 @@ struct mhit_ctx {
   int mom_tma = 1;                        // k_mom fills its interior rings by TMA (test hook: 0)
   int graph_kernels = 0;                  // kernel nodes in a captured step graph
   // 1: the inverse x transform runs fused with the projection (k_xinv_correct); 0: k_fftx_inv +
-  // k_correct; -1 (the default): fused where that is the faster.  Step times of the two without the
-  // phase field, separate / fused: nx = 512 from 8192 x lines on (512x128x64 FP64 232 / 227 us, FP32
-  // 194 / 190, incremental 216 / 207; 512x64x64 117 / 135, 105 / 119, 120 / 131); nx = 256 in FP64 from
-  // 65536 lines on (256^3 849 / 826 us, 256x1024x64 888 / 851; 256x128x128 240 / 244; FP32 always
-  // slower, 256^3 689 / 713).  At 192 points and less, and at 1024^3, where k_correct streams at 96%
-  // of the copy peak, the separate passes are faster.  The fused
+  // k_correct; -1 (the default): fused where that is the faster, from 2^22 cells on at nx = 192, 256
+  // and 512.  Step times without the phase field, separate / fused, FP64, FP32, incremental (us):
+  //   512x128x64   235 / 220, 194 / 185, 216 / 199     512x64x64    118 / 128, 105 / 113, 120 / 125
+  //   256^3        849 / 789, 691 / 664, 785 / 721     256x256x64   234 / 215, 192 / 183, 217 / 202
+  //   256x64x64     73 / 79,   69 / 74,   82 / 86      192^3        399 / 389, 326 / 314, 366 / 348
+  //   192x64x128   100 / 101,  90 / 91,   98 / 99      128^3        123 / 122, 105 / 110, 115 / 117
+  //   64x512x512   858 / 947, 715 / 806, 788 / 908
+  // (at 1024^3, where k_correct streams at 96% of the copy peak, the separate passes win).  The fused
   // pass leaves the pressure in the spectrum only: after such a step p_lazy is set, and whatever
   // reads the pressure or reuses the spectrum first materialises it (materialise_pressure).
   int fuse_xc = -1;
@@ -122,9 +124,7 @@ static bool incremental(const mhit_ctx* c) { return c->prm.poisson == MHIT_POISS
 static bool fused_xc(const mhit_ctx* c) {
   if (refined(c)) return false;
   if (c->fuse_xc >= 0) return c->fuse_xc != 0;
-  const long long lines = (long long)c->g.ny * c->g.nz;
-  if (c->g.nx == 512) return lines >= 8192;
-  return c->g.nx == 256 && c->prm.poisson == MHIT_POISSON_FP64 && lines >= 65536;
+  return c->g.nx >= 192 && c->g.nx <= 512 && c->n >= ((size_t)1 << 22);
 }
 
 static int check_ctx(mhit_ctx* c) {
