@@ -386,6 +386,199 @@ __global__ void __launch_bounds__(MNT, 3) k_mom(const __grid_constant__ MomArgs 
   mom_tile<PHI, true>(a, a.alpha, a.beta, blockIdx.x, blockIdx.y, blockIdx.z, smraw);
 }
 
+// The momentum step of large boxes without the phase field: a block of NTX x NTY cells, two vertically
+// adjacent cells
+// per thread (a: row j, b: row j + 1), which carry in registers what they have read of their columns:
+// u, v, w of planes k-1 and k and the neighbours that one plane's formulas share with the next.  13
+// shared loads per cell instead of the 27 of mom_tile, whose shared-memory pipe is the bound, in two
+// blocks of 256 threads and 124 registers per SM; the same bits.  Against mom_tile: 2508 -> 2315 us at
+// 512^3, 2509 -> 2299 at 1024x512x256, 1273 -> 1156 at 512x512x256, 615 -> 589 at 512x512x128, but 308 ->
+// 326 at 256^3, where the few blocks of half the SM leave some with one, and 11 -> 13 at 16^3: taken
+// from 2^25 cells on (mom_pairs).  With the phase field the pairs spill, and 16 warps per SM are too
+// few (2.72 -> 2.86 ms at 512^3).
+//
+// Rings of u, v, w planes k, k+1 (read) and k+2 (in flight) as in mom_tile, filled by TMA boxes or
+// 16-byte copies one plane ahead; one barrier per plane.
+constexpr int NTX = 32, NTY = 16, NNT = NTX * NTY / 2;
+constexpr int NPX = NTX + 4, NPY = NTY + 2;  // ring plane: x in [-2, T+2), y in [-1, T+1)
+constexpr int NPAIRS = NPY * (NPX / 2), NCP = (NPAIRS + NNT - 1) / NNT;  // 16-byte copies per plane, per thread
+constexpr int NPS = (NPX * NPY * 8 + 127) / 128 * 16;  // doubles of a ring slot
+constexpr unsigned NBYTES = NPX * NPY * 8;
+constexpr int NBLK = 2;                                // resident blocks per SM
+
+struct MomNsSmem {
+  double u[4][NPS], v[4][NPS], w[4][NPS];
+  unsigned long long bar[2];
+};
+
+__global__ void __launch_bounds__(NNT, NBLK) k_mom_ns(const __grid_constant__ MomArgs a) {
+  extern __shared__ __align__(128) unsigned char smraw[];
+  MomNsSmem& S = *reinterpret_cast<MomNsSmem*>(smraw);
+  const Geo& g = a.g;
+  const int nx = g.nx, ny = g.ny, nz = g.nz;
+  const size_t plane = (size_t)nx * ny;
+  const int i0 = blockIdx.x * NTX, j0 = blockIdx.y * NTY;
+  const int k0 = blockIdx.z * a.zchunk, k1 = min(k0 + a.zchunk, nz);
+  const int tid = threadIdx.x;
+
+  // source offsets in the plane of this thread's 16-byte pairs (-1: no pair); pair e is the e-th of
+  // the ring plane, whose rows have no gaps
+  int src[NCP];
+#pragma unroll
+  for (int m = 0; m < NCP; ++m) {
+    const int e = tid + m * NNT, y = e / (NPX / 2), xp = e - y * (NPX / 2);
+    src[m] = e < NPAIRS ? pmod_int(j0 - 1 + y, ny) * nx + pmod_int(i0 - 2 + 2 * xp, nx) : -1;
+  }
+  const bool tma = a.tma && i0 >= 2 && i0 + NTX + 2 <= nx && j0 >= 2 && j0 + NTY + 1 <= ny;
+  const uint32_t bar0 = sm_addr(&S.bar[0]);
+  if (tma && tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0) : "memory");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + 8) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (tma) __syncthreads();
+  // planes m.. of group grp (0: the two of the prologue, then one per plane), as in mom_tile
+  auto issue = [&](int m, int count, int grp) {
+    if (tma) {
+      if (tid != 0) return;
+      const uint32_t bar = bar0 + 8 * (grp & 1);
+      expect_tx(bar, 3 * count * NBYTES);
+      for (int q = m; q < m + count; ++q) {
+        const int slot = (q - k0 + 16) & 3, z = pmod_int(q, nz);
+        tma_box(&S.u[slot][0], &a.tmu, i0 - 2, j0 - 1, z, bar);
+        tma_box(&S.v[slot][0], &a.tmv, i0 - 2, j0 - 1, z, bar);
+        tma_box(&S.w[slot][0], &a.tmw, i0 - 2, j0 - 1, z, bar);
+      }
+    } else {
+      for (int q = m; q < m + count; ++q) {
+        const size_t base = (size_t)pmod_int(q, nz) * plane;
+        const int slot = (q - k0 + 16) & 3;
+#pragma unroll
+        for (int e = 0; e < NCP; ++e)
+          if (src[e] >= 0) {
+            cp16(&S.u[slot][2 * (tid + e * NNT)], a.u + base + src[e]);
+            cp16(&S.v[slot][2 * (tid + e * NNT)], a.v + base + src[e]);
+            cp16(&S.w[slot][2 * (tid + e * NNT)], a.w + base + src[e]);
+          }
+      }
+      __pipeline_commit();
+    }
+  };
+  bool waits_ok = true;
+  // the copies of group grp have landed for everyone, and everyone is done with the plane before
+  auto arrive = [&](int grp) {
+    if (tma) {
+      if (!bar_wait(bar0 + 8 * (grp & 1), (grp >> 1) & 1)) waits_ok = false;
+    } else {
+      __pipeline_wait_prior(0);
+    }
+    __syncthreads();
+  };
+
+  const double mu_ = a.sc->mean[0], mv_ = a.sc->mean[1], mw_ = a.sc->mean[2];
+  const int tx = tid % NTX, ty = 2 * (tid / NTX);
+  const int i = i0 + tx, j = j0 + ty;  // lower cell; j and ny are even
+  const bool own = i < nx && j < ny;
+  const double* t = a.tabs;
+  const double sxi = own ? __ldg(t + i) : 0.0, cxi = own ? __ldg(t + nx + i) : 0.0;
+  double syj[2], cyj[2];
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    syj[e] = own ? __ldg(t + 2 * nx + j + e) : 0.0;
+    cyj[e] = own ? __ldg(t + 2 * nx + ny + j + e) : 0.0;
+  }
+  const double c_adv = -0.25 * g.dxi, c_vis = g.mu * g.ddxi * g.rhoi;  // as in mom_tile
+  const double dta = g.dt * a.alpha, dtb = g.dt * a.beta;
+  const int uq = (ty + 1) * NPX + (tx + 2);  // lower cell in the ring plane
+
+  issue(k0 - 1, 2, 0);
+  arrive(0);
+  if (k0 < k1) issue(k0 + 1, 1, 1);
+  // on entry to plane k: u, v, w of planes k-1 (m) and k (0); u(i+1) and v(j+2) of plane k-1; w(i-1)
+  // and w(j-1) of plane k
+  const double *Um = S.u[3] + uq, *Vm = S.v[3] + uq, *Wm = S.w[3] + uq;  // plane k0-1
+  double uam = Um[0] - mu_, ubm = Um[NPX] - mu_, uaxm = Um[1] - mu_, ubxm = Um[NPX + 1] - mu_;
+  double vam = Vm[0] - mv_, vbm = Vm[NPX] - mv_, vbnm = Vm[2 * NPX] - mv_;
+  double wam = Wm[0] - mw_, wbm = Wm[NPX] - mw_;
+  const double *Uc = S.u[0] + uq, *Vc = S.v[0] + uq, *Wc = S.w[0] + uq;  // plane k0
+  double ua0 = Uc[0] - mu_, ub0 = Uc[NPX] - mu_, va0 = Vc[0] - mv_, vb0 = Vc[NPX] - mv_;
+  double wa0 = Wc[0] - mw_, wb0 = Wc[NPX] - mw_;
+  double waw = Wc[-1] - mw_, wbw = Wc[NPX - 1] - mw_, was = Wc[-NPX] - mw_;
+
+  size_t c = (size_t)k0 * plane + (size_t)(own ? j : 0) * nx + (own ? i : 0);
+#pragma unroll 2
+  for (int k = k0; k < k1; ++k, c += plane) {
+    double ro[2][3] = {};
+    if (own) {
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        ro[e][0] = a.ru[c + (size_t)e * nx];
+        ro[e][1] = a.rv[c + (size_t)e * nx];
+        ro[e][2] = a.rw[c + (size_t)e * nx];
+      }
+    }
+    arrive(k - k0 + 1);  // plane k+1
+    if (k + 1 < k1) issue(k + 2, 1, k - k0 + 2);
+    const int s0 = (k - k0 + 16) & 3, sp = (k - k0 + 17) & 3;
+    const double *U0 = S.u[s0] + uq, *V0 = S.v[s0] + uq, *W0 = S.w[s0] + uq;
+    const double *U1 = S.u[sp] + uq, *V1 = S.v[sp] + uq, *W1 = S.w[sp] + uq;
+    const double uax = U0[1] - mu_, uaw = U0[-1] - mu_, uas = U0[-NPX] - mu_, uasx = U0[-NPX + 1] - mu_;
+    const double vax = V0[1] - mv_, vaw = V0[-1] - mv_, vas = V0[-NPX] - mv_, vbw = V0[NPX - 1] - mv_;
+    const double wax = W0[1] - mw_, wawz = W1[-1] - mw_, wasz = W1[-NPX] - mw_;
+    const double uaz = U1[0] - mu_, vaz = V1[0] - mv_, waz = W1[0] - mw_;
+    const double szk = __ldg(t + 2 * nx + 2 * ny + k), czk = __ldg(t + 2 * nx + 2 * ny + nz + k);
+    auto dsq = [](double a1, double b1) { return __fma_rn(a1, a1, -(b1 * b1)); };
+    auto dpr = [](double a1, double c1, double b1, double d1) { return __fma_rn(a1, c1, -(b1 * d1)); };
+    // the formulas of mom_tile (multi/main.f90:672-714, :787-792) for one cell
+    auto cell = [&](int e, double u0, double uxp, double uxm, double uyp, double uym, double uzp, double uzm, double v0,
+                    double vxp, double vxm, double vyp, double vym, double vzp, double vzm, double w0, double wxp,
+                    double wxm, double wyp, double wym, double wzp, double wzm, double v_imjp, double w_imkp,
+                    double u_ipjm, double w_jmkp, double u_ipkm, double v_jpkm) {
+      const double h11 = dsq(uxp + u0, u0 + uxm);
+      const double h12 = dpr(uyp + u0, vyp + v_imjp, u0 + uym, v0 + vxm);
+      const double h13 = dpr(uzp + u0, wzp + w_imkp, u0 + uzm, w0 + wxm);
+      const double h21 = dpr(uxp + u_ipjm, vxp + v0, u0 + uym, v0 + vxm);
+      const double h22 = dsq(vyp + v0, v0 + vym);
+      const double h23 = dpr(wzp + w_jmkp, vzp + v0, w0 + wym, v0 + vzm);
+      const double h31 = dpr(wxp + w0, uxp + u_ipkm, w0 + wxm, u0 + uzm);
+      const double h32 = dpr(vyp + v_jpkm, wyp + w0, v0 + vzm, w0 + wym);
+      const double h33 = dsq(wzp + w0, w0 + wzm);
+      const double lu = ((uxp + uxm) + (uyp + uym)) + __fma_rn(-6.0, u0, uzp + uzm);
+      const double lv = ((vxp + vxm) + (vyp + vym)) + __fma_rn(-6.0, v0, vzp + vzm);
+      const double lw = ((wxp + wxm) + (wyp + wym)) + __fma_rn(-6.0, w0, wzp + wzm);
+      double ru = __fma_rn(c_adv, (h11 + h12) + h13, c_vis * lu);
+      double rv = __fma_rn(c_adv, (h21 + h22) + h23, c_vis * lv);
+      double rw = __fma_rn(c_adv, (h31 + h32) + h33, c_vis * lw);
+      ru = __fma_rn(g.f3, szk, __fma_rn(g.f2, cyj[e], ru));
+      rv = __fma_rn(g.f1, sxi, __fma_rn(g.f3, czk, rv));
+      rw = __fma_rn(g.f2, syj[e], __fma_rn(g.f1, cxi, rw));
+      const size_t o = c + (size_t)e * nx;
+      a.un[o] = __fma_rn(dta, ru, __fma_rn(-dtb, ro[e][0], u0));
+      a.vn[o] = __fma_rn(dta, rv, __fma_rn(-dtb, ro[e][1], v0));
+      a.wn[o] = __fma_rn(dta, rw, __fma_rn(-dtb, ro[e][2], w0));
+      a.ru[o] = ru;
+      a.rv[o] = rv;
+      a.rw[o] = rw;
+    };
+    if (own)
+      cell(0, ua0, uax, uaw, ub0, uas, uaz, uam, va0, vax, vaw, vb0, vas, vaz, vam, wa0, wax, waw, wb0, was, waz, wam,
+           vbw, wawz, uasx, wasz, uaxm, vbm);
+    // the upper cell's operands are read after the lower cell is done: together they spill
+    asm volatile("" ::: "memory");
+    const double ubx = U0[NPX + 1] - mu_, ubw = U0[NPX - 1] - mu_, ubn = U0[2 * NPX] - mu_, ubz = U1[NPX] - mu_;
+    const double vbx = V0[NPX + 1] - mv_, vbn = V0[2 * NPX] - mv_, vbnw = V0[2 * NPX - 1] - mv_, vbz = V1[NPX] - mv_;
+    const double wbx = W0[NPX + 1] - mw_, wbn = W0[2 * NPX] - mw_, wbwz = W1[NPX - 1] - mw_, wbz = W1[NPX] - mw_;
+    if (own)
+      cell(1, ub0, ubx, ubw, ubn, ua0, ubz, ubm, vb0, vbx, vbw, vbn, va0, vbz, vbm, wb0, wbx, wbw, wbn, wa0, wbz, wbm,
+           vbnw, wbwz, uax, waz, ubxm, vbnm);
+    uam = ua0, ua0 = uaz, uaxm = uax, ubm = ub0, ub0 = ubz, ubxm = ubx;
+    vam = va0, va0 = vaz, vbm = vb0, vb0 = vbz, vbnm = vbn;
+    wam = wa0, wa0 = waz, waw = wawz, was = wasz, wbm = wb0, wb0 = wbz, wbw = wbwz;
+  }
+  __pipeline_wait_prior(0);
+  if (!waits_ok) atomicOr(&const_cast<DevScalars*>(a.sc)->flag, 4);  // as in mom_tile
+}
+
 // The momentum step of many boxes in one launch: persistent blocks (three per SM) take work items
 // (box, tile x, tile y, z chunk) from a device queue until it is empty.  The boxes' arguments live
 // in device memory, so their rings are filled by per-thread copies (no TMA).
@@ -435,35 +628,45 @@ cudaError_t launch_mom_batch(const BatchArgs<MomArgs>& b, bool phi, int nsm, cud
   return cudaGetLastError();
 }
 
-template <bool PHI>
-static cudaError_t launch_mom_t(const MomArgs& a, cudaStream_t st) {
-  const size_t smem = sizeof(MomSmem<PHI>);
-  static int attr_set[64] = {0};
+static bool mom_pairs(const Geo& g) { return (size_t)g.nx * g.ny * g.nz >= (size_t)1 << 25; }
+
+MomBox mom_velocity_box(const Geo& g, bool phi) { return !phi && mom_pairs(g) ? MomBox::VelocityNs : MomBox::Velocity; }
+
+cudaError_t launch_mom(const MomArgs& a, cudaStream_t st) {
+  // 0: with the phase field, 1: without, 2: without, large
+  const int which = a.phi ? 0 : (mom_pairs(a.g) ? 2 : 1);
+  const size_t smem = which == 0 ? sizeof(MomSmem<true>) : (which == 1 ? sizeof(MomSmem<false>) : sizeof(MomNsSmem));
+  auto kern = which == 0 ? k_mom<true> : (which == 1 ? k_mom<false> : k_mom_ns);
+  static int attr_set[64][3] = {};
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev < 64 && !attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(k_mom<PHI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (dev >= 64 || !attr_set[dev][which]) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    attr_set[dev] = 1;
+    if (dev < 64) attr_set[dev][which] = 1;
   }
   MomArgs b = a;
-  b.zchunk = mom_zchunk(a.g, a.zchunk, a.many);
-  k_mom<PHI><<<mom_grid(a.g, b.zchunk), MNT, smem, st>>>(b);
+  if (which == 2) {
+    b.zchunk = a.zchunk > 0 ? a.zchunk : 64;  // the blocks make at least three waves
+    const dim3 grid((a.g.nx + NTX - 1) / NTX, (a.g.ny + NTY - 1) / NTY, (a.g.nz + b.zchunk - 1) / b.zchunk);
+    kern<<<grid, NNT, smem, st>>>(b);
+  } else {
+    b.zchunk = mom_zchunk(a.g, a.zchunk, a.many);
+    kern<<<mom_grid(a.g, b.zchunk), MNT, smem, st>>>(b);
+  }
   return cudaGetLastError();
 }
 
-cudaError_t launch_mom(const MomArgs& a, cudaStream_t st) {
-  return a.phi ? launch_mom_t<true>(a, st) : launch_mom_t<false>(a, st);
-}
-
-int mom_field_map(CUtensorMap* map, const double* field, int nx, int ny, int nz, bool phi) {
+int mom_field_map(CUtensorMap* map, const double* field, int nx, int ny, int nz, MomBox box_of) {
+  static_assert(UPX == PPX && UPX == NPX, "one box width");
+  const int rows = box_of == MomBox::Phi ? PPY : (box_of == MomBox::Velocity ? UPY : NPY);
   EncodeTiledFn enc = tensor_map_encoder();
   if (!enc) return set_error(MHIT_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
-  // x-fastest float64 field; box UPX x UPY (PPX x PPY for phi) x 1 plane.  The row stride nx * 8
+  // x-fastest float64 field; box UPX x rows x 1 plane.  The row stride nx * 8
   // bytes is a multiple of 16 (nx is even) and the box rows are 288 bytes.
   const cuuint64_t dims[3] = {(cuuint64_t)nx, (cuuint64_t)ny, (cuuint64_t)nz};
   const cuuint64_t strides[2] = {(cuuint64_t)nx * 8, (cuuint64_t)nx * ny * 8};
-  const cuuint32_t box[3] = {(cuuint32_t)UPX, (cuuint32_t)(phi ? PPY : UPY), 1};
+  const cuuint32_t box[3] = {(cuuint32_t)UPX, (cuuint32_t)rows, 1};
   const cuuint32_t estr[3] = {1, 1, 1};
   const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, const_cast<double*>(field), dims, strides, box, estr,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,

@@ -132,9 +132,11 @@ cudaError_t launch_mom(const MomArgs& a, cudaStream_t st);
 int mom_zchunk(const Geo& g, int requested, bool many);  // the z chunk launch_mom uses
 dim3 mom_grid(const Geo& g, int zc);           // its tiles: x, y, z chunk
 cudaError_t launch_mom_batch(const BatchArgs<MomArgs>& b, bool phi, int nsm, cudaStream_t st);
-// tensor map of an x-fastest nx*ny*nz float64 field with the ring box of k_mom (36 x 10 for the
-// velocity, 36 x 11 for phi)
-int mom_field_map(CUtensorMap* map, const double* field, int nx, int ny, int nz, bool phi);
+// tensor map of an x-fastest nx*ny*nz float64 field with the ring box of the momentum kernels: u, v, w
+// (36 x 10; 36 x 18 in the kernel of large boxes without the phase field) and phi (36 x 11)
+enum class MomBox { Velocity, Phi, VelocityNs };
+MomBox mom_velocity_box(const Geo& g, bool phi);
+int mom_field_map(CUtensorMap* map, const double* field, int nx, int ny, int nz, MomBox box_of);
 
 // ---------------------------------------------------------------- projection + reductions
 struct CorrectArgs {

@@ -687,11 +687,12 @@ static int init_impl(const mhit_params* p, mhit_ctx* c) {
       MHIT_CUDA_TRY(cudaMemset(c->PHI[i], 0, fb));
     }
   }
+  const MomBox vbox = mom_velocity_box(g, p->phiflag != 0);
   for (int i = 0; i < 2; ++i) {  // the momentum kernel's TMA boxes over each ping-pong buffer
-    if ((rc0 = mom_field_map(&c->tm_u[i], c->U[i], g.nx, g.ny, g.nz, false))) return rc0;
-    if ((rc0 = mom_field_map(&c->tm_v[i], c->V[i], g.nx, g.ny, g.nz, false))) return rc0;
-    if ((rc0 = mom_field_map(&c->tm_w[i], c->W[i], g.nx, g.ny, g.nz, false))) return rc0;
-    if (p->phiflag && (rc0 = mom_field_map(&c->tm_phi[i], c->PHI[i], g.nx, g.ny, g.nz, true))) return rc0;
+    if ((rc0 = mom_field_map(&c->tm_u[i], c->U[i], g.nx, g.ny, g.nz, vbox))) return rc0;
+    if ((rc0 = mom_field_map(&c->tm_v[i], c->V[i], g.nx, g.ny, g.nz, vbox))) return rc0;
+    if ((rc0 = mom_field_map(&c->tm_w[i], c->W[i], g.nx, g.ny, g.nz, vbox))) return rc0;
+    if (p->phiflag && (rc0 = mom_field_map(&c->tm_phi[i], c->PHI[i], g.nx, g.ny, g.nz, MomBox::Phi))) return rc0;
   }
   MHIT_CUDA_TRY(cudaMalloc(&c->RU, fb));
   MHIT_CUDA_TRY(cudaMalloc(&c->RV, fb));

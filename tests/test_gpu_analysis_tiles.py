@@ -37,6 +37,19 @@ def test_labels_of_random_masks(gpu, shape, fill, conn):
         assert np.max(np.abs(got[key] - ref[key])) < 1e-12, key
 
 
+def test_every_masked_cell_is_counted_in_every_call(gpu):
+    n = 256
+    z = np.zeros((n, n, n))
+    with Solver(Params(nx=n, phiflag=1)) as s:
+        s.upload(z, z, z, z)
+        s.init_drops(synth.drop_centres(64, 3), 0.3)
+        mask = int((s.download(("phi",))["phi"] >= 0.5).sum())
+        first = s.label_drops(0.5, 6)["cells"]
+        assert int(first.sum()) == mask
+        for _ in range(30):
+            np.testing.assert_array_equal(s.label_drops(0.5, 6)["cells"], first)
+
+
 @pytest.mark.parametrize("shape", [(16, 16, 16), (32, 64, 16), (192, 16, 64)])
 def test_diagnostics_and_spectrum_of_ragged_boxes(gpu, shape):
     nx, ny, nz = shape

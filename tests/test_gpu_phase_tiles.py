@@ -7,7 +7,7 @@ FP64 evaluation of the oracle's expressions, so the usual 1e-12 of the buffer's 
 import numpy as np
 import pytest
 
-from mhit36_mixedp_b200 import Params, Solver, synth
+from mhit36_mixedp_b200 import Params, Solver, _lib, synth
 from oracle import mhit_oracle as orc
 
 pytestmark = pytest.mark.gpu
@@ -40,4 +40,24 @@ def test_stencil_stages_on_ragged_boxes(gpu, shape, clamp):
         orc.momentum_step(op, st, orc.forcing_tables(op))
         s.run_stage("momentum")
         for f, name in (("un", "u"), ("vn", "v"), ("wn", "w")):
+            assert rel(s.buffer(f), getattr(st, name)) < TOL
+
+
+@pytest.mark.parametrize("tma", [1, 0])
+def test_momentum_of_a_large_box_without_the_phase_field(gpu, tma):
+    """From 2^25 cells on the single-phase momentum step has a kernel of its own; a flat box of that
+    size, its rings filled by TMA boxes (where they need no wrap) and by copies."""
+    nx, ny, nz = 1024, 1024, 32
+    u, v, w = synth.solenoidal_velocity(nx, 3, ny=ny, nz=nz)
+    prm = dict(nx=nx, ny=ny, nz=nz, dt=5e-5, mu=0.004)
+    op = orc.Params(**prm)
+    st = orc.new_state(op, u, v, w)
+    with Solver(Params(**prm)) as s:
+        assert _lib.load().mhit_debug_set_mom_tma(s._ctx, tma) == 0
+        s.upload(u, v, w)
+        s.run_stage("momentum")
+        orc.momentum_step(op, st, orc.forcing_tables(op))
+        for f, name in (("un", "u"), ("vn", "v"), ("wn", "w")):
+            assert rel(s.buffer(f), getattr(st, name)) < TOL
+        for f, name in (("ru", "rhsu_o"), ("rv", "rhsv_o"), ("rw", "rhsw_o")):
             assert rel(s.buffer(f), getattr(st, name)) < TOL
