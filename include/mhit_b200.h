@@ -322,7 +322,7 @@ int mhit_debug_set_mom_tma(mhit_ctx* ctx, int on);
  * transformed into its array only when something reads it: a download, a field file, a
  * checkpoint, a debug read, or a call that reuses the spectrum buffer); 0: the two passes of
  * multi/main.f90:909-912 and :942-1003 run apart; -1 (the default): fused where it is the faster
- * (nx = 512).  The refinement sweep always runs them apart.  The results agree to rounding (a
+ * (2^22 cells and more at nx = 192, 256, 512).  The refinement sweep always runs them apart.  The results agree to rounding (a
  * test compares). */
 int mhit_debug_set_fused_projection(mhit_ctx* ctx, int on);
 long long mhit_debug_buffer_len(mhit_ctx* ctx, int which);
