@@ -1924,6 +1924,10 @@ static int ens_check_flags(mhit_ensemble* e, bool stepped) {
     int rc;
     if (!stepped && (rc = fetch_scalars(e->box[b]))) return rc;
     const int flag = e->box[b]->sc_host->flag;
+    // first: what a wait that ran out leaves behind may be NaN or a large Courant number too
+    if (flag & 4)
+      return set_error(MHIT_ERR_TIMEOUT,
+                       "a bounded wait ran out in ensemble box " + std::to_string(b) + " (results invalid)");
     if (flag & 1) return set_error(MHIT_ERR_NAN, "NaN in the velocity field of ensemble box " + std::to_string(b));
     if (flag & 2) return set_error(MHIT_ERR_CFL, "CFL > 7 in ensemble box " + std::to_string(b));
   }

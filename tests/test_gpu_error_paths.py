@@ -8,6 +8,8 @@
   out (a corrupted parent chain would otherwise loop).  The test hook lowers the bound to 1, so
   ordinary chains of a drop run out; ``mhit_label_drops`` must return MHIT_ERR_STATE, and with the
   default bound the same call must succeed.
+* A bounded wait inside a kernel that runs out sets bit 2 of the flag word, which stays set.  The
+  tests set the bit through a checkpoint, whose header holds the word, so no wait has to run out.
 """
 import ctypes
 import math
@@ -15,7 +17,8 @@ import math
 import numpy as np
 import pytest
 
-from mhit36_mixedp_b200 import MhitCFLError, MhitStateError, Params, Solver, _lib, synth
+from mhit36_mixedp_b200 import Ensemble, MhitCFLError, MhitStateError, Params, Solver, _lib, synth
+from mhit36_mixedp_b200.api import MhitTimeoutError
 
 pytestmark = pytest.mark.gpu
 
@@ -71,3 +74,33 @@ def test_label_bound_exhaustion_is_an_error_status(gpu):
         again = s.label_drops(0.5, 6)
         np.testing.assert_array_equal(again["cells"], ok["cells"])
         assert lib.mhit_debug_set_label_bound(s._ctx, ctypes.c_longlong(-1)) == _lib.MHIT_ERR_ARG
+
+
+FLAG_OFFSET = 48 + 40  # CkptHeader, then mean[3], gumax, cfl of the device scalars
+
+
+def raise_wait_flag(solver, path):
+    """Set bit 2 of the flag word of a context's device scalars, the state otherwise unchanged."""
+    solver.write_checkpoint(path)
+    with open(path, "r+b") as f:
+        f.seek(FLAG_OFFSET)
+        assert f.read(4) == b"\0\0\0\0"
+        f.seek(FLAG_OFFSET)
+        f.write(b"\4\0\0\0")
+    solver.read_checkpoint(path)
+    assert solver.diagnostics()["flags"] == 4
+
+
+@pytest.mark.parametrize("batched", [True, False])
+def test_exhausted_wait_stops_the_ensemble(gpu, tmp_path, batched):
+    n = 16
+    u, v, w = synth.solenoidal_velocity(n, 0)
+    with Ensemble([Params(nx=n, dt=5e-4)] * 3) as e:
+        e.set_batched(batched)
+        for s in e.boxes:
+            s.upload(u, v, w)
+        e.step(2)
+        raise_wait_flag(e.boxes[1], str(tmp_path / "box.ckp"))
+        for nsteps in (0, 1):
+            with pytest.raises(MhitTimeoutError, match="box 1"):
+                e.step(nsteps)
