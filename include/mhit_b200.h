@@ -37,7 +37,7 @@ extern "C" {
 #define MHIT_ERR_CFL (-4)      /* CFL > 7 after a step: the reference stops (multi/main.f90:1006) */
 #define MHIT_ERR_IO (-5)       /* file missing, short read or write */
 #define MHIT_ERR_STATE (-6)    /* call out of order (e.g. particles on a context without them) */
-#define MHIT_ERR_TIMEOUT (-7)  /* a bounded wait inside a kernel ran out (tensor-core z solve) */
+#define MHIT_ERR_TIMEOUT (-7)  /* a bounded wait ran out (momentum step, tensor-core z solve) */
 
 /* Poisson precision (multi/main.f90:844,853-912) */
 #define MHIT_POISSON_FP64 0    /* the intended FP64 solve of the main branch */

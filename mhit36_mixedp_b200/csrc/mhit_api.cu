@@ -892,7 +892,8 @@ int mhit_step(mhit_ctx* c, int nsteps) {
   if (nsteps > 0) MHIT_CUDA_TRY(cudaStreamSynchronize(c->st));
   else if ((rc = fetch_scalars(c))) return rc;
   if (c->sc_host->flag & 4)
-    return set_error(MHIT_ERR_TIMEOUT, "the tensor-core z solve gave up on a bounded wait (results invalid)");
+    return set_error(MHIT_ERR_TIMEOUT,
+                     "a bounded wait of the momentum step or of the tensor-core z solve ran out (results invalid)");
   if (c->sc_host->flag & 1) return set_error(MHIT_ERR_NAN, "NaN in the velocity field");
   if (c->sc_host->flag & 2) {
     char b[128];
@@ -1927,7 +1928,8 @@ static int ens_check_flags(mhit_ensemble* e, bool stepped) {
     // first: what a wait that ran out leaves behind may be NaN or a large Courant number too
     if (flag & 4)
       return set_error(MHIT_ERR_TIMEOUT,
-                       "a bounded wait ran out in ensemble box " + std::to_string(b) + " (results invalid)");
+                       "a bounded wait of the momentum step or of the tensor-core z solve ran out in ensemble box " +
+                           std::to_string(b) + " (results invalid)");
     if (flag & 1) return set_error(MHIT_ERR_NAN, "NaN in the velocity field of ensemble box " + std::to_string(b));
     if (flag & 2) return set_error(MHIT_ERR_CFL, "CFL > 7 in ensemble box " + std::to_string(b));
   }

@@ -104,3 +104,17 @@ def test_exhausted_wait_stops_the_ensemble(gpu, tmp_path, batched):
         for nsteps in (0, 1):
             with pytest.raises(MhitTimeoutError, match="box 1"):
                 e.step(nsteps)
+
+
+def test_exhausted_wait_is_not_blamed_on_one_kernel(gpu, tmp_path):
+    """The momentum step's copies and the tensor-core z solve raise the same bit; this context has
+    no tensor-core solve."""
+    n = 16
+    u, v, w = synth.solenoidal_velocity(n, 0)
+    with Solver(Params(nx=n, dt=5e-4)) as s:
+        s.upload(u, v, w)
+        s.step(2)
+        raise_wait_flag(s, str(tmp_path / "box.ckp"))
+        for nsteps in (0, 1):
+            with pytest.raises(MhitTimeoutError, match="momentum"):
+                s.step(nsteps)
