@@ -61,3 +61,29 @@ def test_momentum_of_a_large_box_without_the_phase_field(gpu, tma):
             assert rel(s.buffer(f), getattr(st, name)) < TOL
         for f, name in (("ru", "rhsu_o"), ("rv", "rhsv_o"), ("rw", "rhsw_o")):
             assert rel(s.buffer(f), getattr(st, name)) < TOL
+
+
+def test_phase_field_at_the_ends_of_the_logarithm(gpu):
+    """Without the clamp, phi = -1e-16 makes psi = log(0) = -inf and a smaller one NaN, as in the
+    reference; phi = 0, 1 and beyond 1 stay finite.  The stage must give NaN where the oracle does (the
+    normal of an infinite psi difference) and the oracle's values everywhere else."""
+    n = 32
+    u, v, w = synth.solenoidal_velocity(n, 3)
+    z, y, x = np.meshgrid(*(np.arange(n) * 2 * np.pi / n,) * 3, indexing="ij")
+    dx = 2 * np.pi / n
+    phi = 0.5 * (1 - np.tanh((np.cos(x + 0.1) + np.cos(y + 0.13) + np.cos(z + 0.17)) / (2 * dx)))
+    for q, val in enumerate((-1e-16, -1e-15, -0.5, 0.0, 1.0, 1.0 + 2.0**-52, 1.5, 1e-300, 1e-17, 1.0 - 2.0**-53)):
+        phi[16, 3 * q + 1, 7] = val
+    op = orc.Params(nx=n, ny=n, nz=n, dt=2e-4, phiflag=1)
+    st = orc.new_state(op, u, v, w, phi=phi)
+    with np.errstate(all="ignore"):
+        orc.phase_step(op, st)
+    bad = np.isnan(st.rhsphi_o)
+    assert 0 < bad.sum() < bad.size // 8
+    with Solver(Params(nx=n, dt=2e-4, phiflag=1)) as s:
+        s.upload(u, v, w, phi)
+        s.run_stage("phase")
+        for f, name in (("rphi", "rhsphi_o"), ("phin", "phi")):
+            got, ref = s.buffer(f), getattr(st, name)
+            np.testing.assert_array_equal(np.isnan(got), np.isnan(ref))
+            assert rel(got[~bad], ref[~bad]) < TOL, f
