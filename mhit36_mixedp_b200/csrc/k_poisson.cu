@@ -515,6 +515,10 @@ static cudaError_t launch_xinv_m(const PoissonArgs& a, cudaStream_t st) {
 
 template <typename T, int N, int MODE>
 static cudaError_t launch_cols_n(const PoissonArgs& a, int axis, cudaStream_t st) {
+  // the tables behind twy and twz are those of modes 0 and 2 (fft_schedule)
+  static_assert(std::is_same_v<typename ColSched<T, N, 0>::S, typename ColSched<T, N, 1>::S>, "one y schedule");
+  static_assert(sizeof(T) == 4 || std::is_same_v<typename ColSched<T, N, 0>::S, typename ColSched<T, N, 2>::S>,
+                "one FP64 schedule");
   // the FP64 256-point z solve runs faster staged in shared memory (measured at 256^3: 0.105 vs
   // 0.113 ms; FP32, three blocks per SM: 0.066 vs 0.064 ms); every other pass and size register-staged
   constexpr bool staged = MODE == 2 && N == 256 && sizeof(T) == 8;
@@ -617,7 +621,11 @@ static cudaError_t poisson_stage_t(const PoissonArgs& a, int stage, cudaStream_t
       return launch_cols<T, 2>(a, 2, st);
     case PSTAGE_YINV: return launch_cols<T, 1>(a, 1, st);
     case PSTAGE_XINV: return launch_xinv<T>(a, st);
-    case PSTAGE_ZFWD: return launch_cols<T, 0>(a, 2, st);
+    case PSTAGE_ZFWD:
+      // The z table holds the stage twiddles of the solve's schedule (MODE 2).  In FP64 the single
+      // transforms share it; the FP32 ones of 512 and 1024 points do not.
+      if constexpr (sizeof(T) == 8) return launch_cols<T, 0>(a, 2, st);
+      break;
   }
   return cudaErrorInvalidValue;
 }
