@@ -47,21 +47,34 @@ namespace mhit {
 // take 2.01 ms, two 32 x 12 blocks per SM 2.29 ms (without the fetch).  The branch-free log_ratio and
 // rsqrt_fast are what lets the two chains interleave: with CUDA's log and rsqrt, whose special cases
 // branch, this layout takes 2.66 ms where it takes 2.09 and the one-cell layout 2.41 (one box).
-constexpr int PTX = 32, PTY = 24;  // output cells per block in x, y
-constexpr int PMINB = 1;           // resident blocks per SM
-constexpr int PHX = PTX + 4, PHY = PTY + 4;  // positions with the halo of 2
-constexpr int PPOS = PHX * PHY;              // positions of a shared plane
-constexpr int PNT = PHX * PHY / 2;           // threads per block: one per pair of rows
-constexpr int PNO = PTX * PTY / 2;           // threads with two output cells
-constexpr int PNF = PNO + 2 * PTX + 4 + 2 * (PTY / 2);  // ... plus those that evaluate F on the halo of 1
+template <int TX, int TY> struct PhaseTile {
+  static constexpr int PTX = TX, PTY = TY;             // output cells per block in x, y
+  static constexpr int PHX = PTX + 4, PHY = PTY + 4;   // positions with the halo of 2
+  static constexpr int PPOS = PHX * PHY;               // positions of a shared plane
+  static constexpr int PNT = PHX * PHY / 2;            // threads per block: one per pair of rows
+  static constexpr int PNO = PTX * PTY / 2;            // threads with two output cells
+  static constexpr int PNF = PNO + 2 * PTX + 4 + 2 * (PTY / 2);  // ... plus those that evaluate F on the halo of 1
+  // one plane of the output cells' u (one column more), v (one row more), w(k+1) and rhs_o in shared
+  // memory, fetched with cp.async one plane ahead
+  static constexpr int PUX = PTX + 2;
+  static constexpr int PSU = 0, PSV = PSU + PTY * PUX, PSW = PSV + (PTY + 1) * PTX, PSR = PSW + PTY * PTX,
+                       PSTG = PSR + PTY * PTX;
+  // psi, phi, Fx, Fy and the staged fields, twice each
+  static constexpr size_t PSMEM = sizeof(double) * (8 * PPOS + 2 * PSTG);
+};
+// The tiles above, and two of 16 rows for the boxes of 16 or 32 rows, where a third to a half of 24-row
+// tiles lies outside the box: 48 cells wide (520 threads, 96 registers) from nx = 192 on, where the
+// last tile of a row loses little, 32 wide (360 threads) below.  us with 24-row, 32 x 16, 48 x 16 tiles:
+//   1024x32x1024 695, 570, 528   512x16x512 96, 83, 78   192x32x1024 139, 116, 107
+//   128x32x128    21,  18,  19   64x32x512  31, 25, 31   32^3         12,  11,  13
+// and (whole steps) 16 boxes of 64x32x64 226, 214, 226, 8 of 256x32x256 1459, 1401, 1372.  At 64 rows
+// 24-row tiles lose an eighth and take 76 against 82 us at 256x64x256 (32 x 16).
+using Tall = PhaseTile<32, 24>;
+using Flat = PhaseTile<32, 16>;
+using Wide = PhaseTile<48, 16>;
+constexpr int PMINB = 1;    // resident blocks per SM
 constexpr int PUNROLL = 2;  // two-plane bodies per loop iteration (1: 2.07 ms at 512^3)
-// one plane of the output cells' u (one column more), v (one row more), w(k+1) and rhs_o in shared
-// memory, fetched with cp.async one plane ahead
-constexpr int PUX = PTX + 2;
-constexpr int PSU = 0, PSV = PSU + PTY * PUX, PSW = PSV + (PTY + 1) * PTX, PSR = PSW + PTY * PTX,
-              PSTG = PSR + PTY * PTX;
-constexpr size_t PSMEM = sizeof(double) * (8 * PPOS + 2 * PSTG);  // psi, phi, Fx, Fy and the staged fields, twice each
-constexpr int PZC = 64;                      // default z planes per block
+constexpr int PZC = 64;      // default z planes per block
 constexpr double ENUM = 1.0e-16;
 constexpr double TNORM = 1.0 / (1.0 + 2.0 * ENUM);
 
@@ -119,9 +132,11 @@ __device__ __forceinline__ int pmodi(int x, int n) {
 
 // One z column of PTX x PTY cells, tile (bx, by), chunk bz, of the box a; dta, dtb = dt alpha,
 // dt beta of the AB2 update.
-template <bool CLAMP>
+template <bool CLAMP, typename L>
 __device__ __forceinline__ void phase_tile(const PhaseArgs& a, double dta, double dtb, int bx, int by, int bz,
                                            unsigned char* smraw) {
+  constexpr int PTX = L::PTX, PTY = L::PTY, PHX = L::PHX, PHY = L::PHY, PPOS = L::PPOS, PNO = L::PNO, PNF = L::PNF;
+  constexpr int PUX = L::PUX, PSU = L::PSU, PSV = L::PSV, PSW = L::PSW, PSR = L::PSR, PSTG = L::PSTG;
   // thread -> column hx and row pair (rows 2 r, 2 r + 1) of the (PHX x PHY) grid of the tile with
   // its halo: first the output pairs (whole warps), then the pairs that add F on the halo of 1
   // (bottom and top row pair, of which only the inner row does; columns 1 and PTX + 2), then the
@@ -327,18 +342,18 @@ __device__ __forceinline__ void phase_tile(const PhaseArgs& a, double dta, doubl
   }
 }
 
-template <bool CLAMP>
-__global__ void __launch_bounds__(PNT, PMINB) k_phase(const __grid_constant__ PhaseArgs a) {
+template <bool CLAMP, typename L>
+__global__ void __launch_bounds__(L::PNT, PMINB) k_phase(const __grid_constant__ PhaseArgs a) {
   extern __shared__ __align__(16) unsigned char smraw[];
-  phase_tile<CLAMP>(a, a.dta, a.dtb, blockIdx.x, blockIdx.y, blockIdx.z, smraw);
+  phase_tile<CLAMP, L>(a, a.dta, a.dtb, blockIdx.x, blockIdx.y, blockIdx.z, smraw);
 }
 
 // The phase step of many boxes in one launch: persistent blocks (one per SM) take work items
 // (box, tile x, tile y, z chunk) from a device queue until it is empty.  A box's arguments
 // (including its resolved z chunk) come from b.args; alpha, beta are the step's.  The boxes of
 // one launch share the psi clamp (CLAMP).
-template <bool CLAMP>
-__global__ void __launch_bounds__(PNT, PMINB) k_phase_batch(const __grid_constant__ BatchArgs<PhaseArgs> b) {
+template <bool CLAMP, typename L>
+__global__ void __launch_bounds__(L::PNT, PMINB) k_phase_batch(const __grid_constant__ BatchArgs<PhaseArgs> b) {
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ int s_item;
   for (;;) {
@@ -349,13 +364,23 @@ __global__ void __launch_bounds__(PNT, PMINB) k_phase_batch(const __grid_constan
     if (it >= b.nitems) break;
     const int4 w = b.items[it];
     const PhaseArgs& a = b.args[w.x];
-    phase_tile<CLAMP>(a, a.g.dt * b.alpha, a.g.dt * b.beta, w.y, w.z, w.w, smraw);
+    phase_tile<CLAMP, L>(a, a.g.dt * b.alpha, a.g.dt * b.beta, w.y, w.z, w.w, smraw);
   }
+}
+
+PhaseTiles phase_tiles(const Geo& g) {
+  return g.ny > 32 ? PhaseTiles::Tall : (g.nx < 192 ? PhaseTiles::Flat : PhaseTiles::Wide);
+}
+
+// f(tile) of the box's tiles
+template <typename F> static auto with_tiles(PhaseTiles t, F f) {
+  return t == PhaseTiles::Tall ? f(Tall{}) : (t == PhaseTiles::Flat ? f(Flat{}) : f(Wide{}));
 }
 
 int phase_zchunk(const Geo& g, int requested, bool many) {
   if (requested > 0) return requested;
-  const long long cols = (long long)((g.nx + PTX - 1) / PTX) * ((g.ny + PTY - 1) / PTY);
+  const dim3 t = phase_grid(g, g.nz);
+  const long long cols = (long long)t.x * t.y;
   if (many) {
     // one of many boxes that share the chip: long chunks, whose four planes of warm-up cost least
     if (cols * ((g.nz + 255) / 256) >= 6 * 148) return 256;
@@ -371,23 +396,30 @@ int phase_zchunk(const Geo& g, int requested, bool many) {
 }
 
 dim3 phase_grid(const Geo& g, int zc) {
-  return dim3((g.nx + PTX - 1) / PTX, (g.ny + PTY - 1) / PTY, (g.nz + zc - 1) / zc);
+  return with_tiles(phase_tiles(g), [&](auto t) {
+    return dim3((g.nx + t.PTX - 1) / t.PTX, (g.ny + t.PTY - 1) / t.PTY, (g.nz + zc - 1) / zc);
+  });
 }
 
-cudaError_t launch_phase_batch(const BatchArgs<PhaseArgs>& b, bool clamp, int nsm, cudaStream_t st) {
-  constexpr size_t smem = PSMEM;
-  auto kern = clamp ? k_phase_batch<true> : k_phase_batch<false>;
+template <typename L>
+static cudaError_t launch_batch(const BatchArgs<PhaseArgs>& b, bool clamp, int nsm, cudaStream_t st) {
+  constexpr size_t smem = L::PSMEM;
+  auto kern = clamp ? k_phase_batch<true, L> : k_phase_batch<false, L>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(b.counter, 0, sizeof(int), st);
   if (e != cudaSuccess) return e;
-  kern<<<b.nitems < nsm ? b.nitems : nsm, PNT, smem, st>>>(b);
+  kern<<<b.nitems < nsm ? b.nitems : nsm, L::PNT, smem, st>>>(b);
   return cudaGetLastError();
 }
 
-cudaError_t launch_phase(const PhaseArgs& a, cudaStream_t st) {
-  constexpr size_t smem = PSMEM;
-  auto kern = a.clamp ? k_phase<true> : k_phase<false>;
+cudaError_t launch_phase_batch(const BatchArgs<PhaseArgs>& b, PhaseTiles tiles, bool clamp, int nsm, cudaStream_t st) {
+  return with_tiles(tiles, [&](auto t) { return launch_batch<decltype(t)>(b, clamp, nsm, st); });
+}
+
+template <typename L> static cudaError_t launch_one(const PhaseArgs& a, cudaStream_t st) {
+  constexpr size_t smem = L::PSMEM;
+  auto kern = a.clamp ? k_phase<true, L> : k_phase<false, L>;
   static int attr_set[64][2] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -402,8 +434,12 @@ cudaError_t launch_phase(const PhaseArgs& a, cudaStream_t st) {
   b.zchunk = phase_zchunk(a.g, a.zchunk, a.many);
   const int zc = b.zchunk;
   if (zc % 2 || a.g.nz % 2) return cudaErrorInvalidValue;  // the plane loop runs two planes at a time
-  kern<<<phase_grid(a.g, zc), PNT, smem, st>>>(b);
+  kern<<<phase_grid(a.g, zc), L::PNT, smem, st>>>(b);
   return cudaGetLastError();
+}
+
+cudaError_t launch_phase(const PhaseArgs& a, cudaStream_t st) {
+  return with_tiles(phase_tiles(a.g), [&](auto t) { return launch_one<decltype(t)>(a, st); });
 }
 
 }  // namespace mhit

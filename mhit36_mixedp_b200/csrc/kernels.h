@@ -109,7 +109,9 @@ template <typename A> struct BatchArgs {
 };
 int phase_zchunk(const Geo& g, int requested, bool many);  // the z chunk launch_phase uses
 dim3 phase_grid(const Geo& g, int zc);           // its tiles: x, y, z chunk
-cudaError_t launch_phase_batch(const BatchArgs<PhaseArgs>& b, bool clamp, int nsm, cudaStream_t st);
+enum class PhaseTiles { Tall, Flat, Wide };
+PhaseTiles phase_tiles(const Geo& g);            // ... of this shape; the boxes of one batched launch share it
+cudaError_t launch_phase_batch(const BatchArgs<PhaseArgs>& b, PhaseTiles tiles, bool clamp, int nsm, cudaStream_t st);
 
 // ---------------------------------------------------------------- momentum
 struct MomArgs {

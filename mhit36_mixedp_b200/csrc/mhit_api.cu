@@ -1693,6 +1693,7 @@ struct mhit_ensemble {
   int* d_counters = nullptr;  // two queue counters per class
   struct Class {
     int p0, np, m0, nm;       // offset and count of the class's phase and momentum items
+    PhaseTiles tiles;         // of its phase items
   };
   std::vector<Class> cls;     // largest boxes first
   std::vector<int> box_cls;   // class of each box
@@ -1728,18 +1729,20 @@ static void ens_free_batch(mhit_ensemble* e) {
 }
 
 // Device copies of every box's phase and momentum arguments (both parities; the step's alpha,
-// beta come with the launch) and the work items of each class of equal-size boxes, the classes
-// largest boxes first.
+// beta come with the launch) and the work items of each class of boxes of equal cell count and phase
+// tiles, the classes largest boxes first.
 static int ens_prepare_batch(mhit_ensemble* e) {
   if (e->batch_ready) return MHIT_OK;
   ens_free_batch(e);
-  std::vector<size_t> sizes;
+  using Key = std::pair<size_t, PhaseTiles>;  // a class: cells, tiles of the phase step
+  auto key = [](const mhit_ctx* c) { return Key(c->n, phase_tiles(c->g)); };
+  std::vector<Key> keys;
   for (const mhit_ctx* c : e->box)
-    if (std::find(sizes.begin(), sizes.end(), c->n) == sizes.end()) sizes.push_back(c->n);
-  std::sort(sizes.begin(), sizes.end(), std::greater<size_t>());
+    if (std::find(keys.begin(), keys.end(), key(c)) == keys.end()) keys.push_back(key(c));
+  std::sort(keys.begin(), keys.end(), std::greater<Key>());
   e->box_cls.assign(e->nbox, 0);
   for (int b = 0; b < e->nbox; ++b)
-    e->box_cls[b] = (int)(std::find(sizes.begin(), sizes.end(), e->box[b]->n) - sizes.begin());
+    e->box_cls[b] = (int)(std::find(keys.begin(), keys.end(), key(e->box[b])) - keys.begin());
   std::vector<int4> pit, mit;
   std::vector<PhaseArgs> pa[2];
   std::vector<MomArgs> ma[2];
@@ -1755,8 +1758,8 @@ static int ens_prepare_batch(mhit_ensemble* e) {
       ma[par].push_back(m);
     }
   }
-  for (size_t k = 0; k < sizes.size(); ++k) {
-    mhit_ensemble::Class cl{(int)pit.size(), 0, (int)mit.size(), 0};
+  for (size_t k = 0; k < keys.size(); ++k) {
+    mhit_ensemble::Class cl{(int)pit.size(), 0, (int)mit.size(), 0, keys[k].second};
     for (int b = 0; b < e->nbox; ++b) {
       if (e->box_cls[b] != (int)k) continue;
       const mhit_ctx* c = e->box[b];
@@ -1846,7 +1849,7 @@ static int ens_enqueue(mhit_ensemble* e, double alpha, double beta, int cur) {
       cudaStream_t lane = e->lanes[e->nlanes - 1 - (int)(k % e->nlanes)];
       if (cl.np) {
         BatchArgs<PhaseArgs> pb{e->d_pargs[cur], e->d_pitems + cl.p0, cl.np, e->d_counters + 2 * k, alpha, beta};
-        MHIT_CUDA_TRY(launch_phase_batch(pb, e->box[0]->prm.acdi_clamp != 0, e->nsm, lane));
+        MHIT_CUDA_TRY(launch_phase_batch(pb, cl.tiles, e->box[0]->prm.acdi_clamp != 0, e->nsm, lane));
       }
       BatchArgs<MomArgs> mb{e->d_margs[cur], e->d_mitems + cl.m0, cl.nm, e->d_counters + 2 * k + 1, alpha, beta};
       MHIT_CUDA_TRY(launch_mom_batch(mb, e->box[0]->prm.phiflag != 0, e->nsm, lane));

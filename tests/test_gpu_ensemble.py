@@ -137,3 +137,26 @@ def test_batched_schedule_matches_lanes_and_standalone(gpu, phiflag):
             for k in ref:
                 np.testing.assert_array_equal(got[mode][b][k], ref[k], err_msg=f"{mode} box {b} {k}")
 
+
+
+def test_batched_boxes_of_one_size_and_unequal_shapes(gpu):
+    """Boxes of equal cell counts whose phase steps run on different tiles (64, 32 and 16 rows, long and
+    short ones): the bits of the standalone boxes."""
+    shapes = [(64, 64, 16), (64, 16, 64), (256, 16, 16), (32, 32, 64), (16, 256, 16)]
+    cases = []
+    for b, (nx, ny, nz) in enumerate(shapes):
+        prm = Params(nx=nx, ny=ny, nz=nz, dt=2e-4, mu=0.004, sigma=0.4, phiflag=1, acdi_clamp=1)
+        u, v, w = synth.solenoidal_velocity(nx, 300 + b, ny=ny, nz=nz)
+        z, y, x = np.meshgrid(*(np.arange(n) * 2 * np.pi / n for n in (nz, ny, nx)), indexing="ij")
+        phi = 0.5 * (1 - np.tanh((np.cos(x + 0.1) + np.cos(y + 0.13) + np.cos(z + 0.17)) * nx / (4 * np.pi)))
+        cases.append((prm, u, v, w, phi))
+    with Ensemble([c[0] for c in cases]) as ens:
+        assert ens.tuning()["batched"]
+        for box, (prm, u, v, w, phi) in zip(ens.boxes, cases):
+            box.upload(u, v, w, phi)
+        ens.step(4)
+        got = [box.download() for box in ens.boxes]
+    for b, (prm, u, v, w, phi) in enumerate(cases):
+        ref = standalone(prm, u, v, w, phi, 4)
+        for k in ref:
+            np.testing.assert_array_equal(got[b][k], ref[k], err_msg=f"box {b} {k}")

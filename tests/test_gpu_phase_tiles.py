@@ -19,7 +19,8 @@ def rel(a, b):
 
 
 @pytest.mark.parametrize("clamp", [0, 1])
-@pytest.mark.parametrize("shape", [(16, 16, 16), (16, 64, 16), (64, 16, 128), (192, 64, 128), (32, 192, 64), (64, 128, 16)])
+@pytest.mark.parametrize("shape", [(16, 16, 16), (16, 64, 16), (64, 16, 128), (192, 64, 128), (32, 192, 64), (64, 128, 16),
+                                   (128, 32, 64), (192, 16, 32), (256, 32, 16)])
 def test_stencil_stages_on_ragged_boxes(gpu, shape, clamp):
     nx, ny, nz = shape
     dx = 2 * np.pi / nx
