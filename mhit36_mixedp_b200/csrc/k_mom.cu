@@ -25,6 +25,8 @@
 // u = u - gumean (:977-981) done lazily.
 #include <cuda_pipeline.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.h"
 
@@ -598,18 +600,22 @@ __global__ void __launch_bounds__(MNT, 3) k_mom_batch(const __grid_constant__ Ba
   }
 }
 
-int mom_zchunk(const Geo& g, int requested, bool many) {
+int mom_zchunk(const Geo& g, int requested, double share) {
   if (requested > 0) return requested;
-  const long long cols = (long long)((g.nx + MTX - 1) / MTX) * ((g.ny + MTY - 1) / MTY);
+  // the columns of all boxes that share the chip, as in phase_zchunk
+  const long long cols = (long long)(((g.nx + MTX - 1) / MTX) * ((g.ny + MTY - 1) / MTY) * share);
   // 64 planes where that leaves eight waves of three blocks on each of the 148 SMs (2.896 against
-  // 2.928 ms at 512^3), MZC for one of many boxes that share the chip.
+  // 2.928 ms at 512^3).
   if (cols * ((g.nz + 63) / 64) >= 8 * 148 * 3) return 64;
-  if (many) return MZC;
   // Smaller grids: the fewest planes in sequence, as k_phase, with three blocks per SM and four
   // planes' time to fill the rings.  Measured, chunk of 32 -> the rule's: 64^3 33 -> 14 us (4
   // planes), 128^3 55 -> 51 us (22), 192x64x128 60 -> 48 us (16), 256^3 unchanged (52 planes).
+  // In an ensemble at most MZC: the queue of the batched launch wants items to balance with (16 boxes of
+  // 192x32x192, steps: 1583 us, with the rule's 192 planes 1634), and shorter where there are few
+  // (16 boxes of 64^3 405 -> 377 us, 4 of 64^3 142 -> 126).
   // Results do not depend on the chunk.
-  return best_zchunk(g.nz, cols, 3 * 148, 4);
+  const int zc = best_zchunk(g.nz, cols, 3 * 148, 4);
+  return share > 1.0 ? std::min(zc, MZC) : zc;
 }
 
 dim3 mom_grid(const Geo& g, int zc) {
@@ -651,7 +657,7 @@ cudaError_t launch_mom(const MomArgs& a, cudaStream_t st) {
     const dim3 grid((a.g.nx + NTX - 1) / NTX, (a.g.ny + NTY - 1) / NTY, (a.g.nz + b.zchunk - 1) / b.zchunk);
     kern<<<grid, NNT, smem, st>>>(b);
   } else {
-    b.zchunk = mom_zchunk(a.g, a.zchunk, a.many);
+    b.zchunk = mom_zchunk(a.g, a.zchunk, a.share);
     kern<<<mom_grid(a.g, b.zchunk), MNT, smem, st>>>(b);
   }
   return cudaGetLastError();

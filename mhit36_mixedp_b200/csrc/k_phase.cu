@@ -74,7 +74,6 @@ using Flat = PhaseTile<32, 16>;
 using Wide = PhaseTile<48, 16>;
 constexpr int PMINB = 1;    // resident blocks per SM
 constexpr int PUNROLL = 2;  // two-plane bodies per loop iteration (1: 2.07 ms at 512^3)
-constexpr int PZC = 64;      // default z planes per block
 constexpr double ENUM = 1.0e-16;
 constexpr double TNORM = 1.0 / (1.0 + 2.0 * ENUM);
 
@@ -170,7 +169,7 @@ __device__ __forceinline__ void phase_tile(const PhaseArgs& a, double dta, doubl
   const int nx = g.nx, ny = g.ny, nz = g.nz;
   const int plane = nx * ny, ntot = plane * nz;
   const int i0 = bx * PTX, j0 = by * PTY;
-  const int zc = a.zchunk > 0 ? a.zchunk : PZC;
+  const int zc = a.zchunk;
   const int k0 = bz * zc, k1 = min(k0 + zc, nz);
   const int i = i0 - 2 + hx, j = j0 - 2 + 2 * r;  // lower cell; j and ny are even
   const int ic = pmodi(i, nx), jc = pmodi(j, ny);
@@ -377,22 +376,20 @@ template <typename F> static auto with_tiles(PhaseTiles t, F f) {
   return t == PhaseTiles::Tall ? f(Tall{}) : (t == PhaseTiles::Flat ? f(Flat{}) : f(Wide{}));
 }
 
-int phase_zchunk(const Geo& g, int requested, bool many) {
+int phase_zchunk(const Geo& g, int requested, double share) {
   if (requested > 0) return requested;
   const dim3 t = phase_grid(g, g.nz);
   const long long cols = (long long)t.x * t.y;
-  if (many) {
-    // one of many boxes that share the chip: long chunks, whose four planes of warm-up cost least
-    if (cols * ((g.nz + 255) / 256) >= 6 * 148) return 256;
-    return cols * ((g.nz + 127) / 128) >= 8 * 148 ? 128 : PZC;
-  }
   // The even chunk with the fewest planes in sequence on an SM: waves of one block on each of the
   // 148 SMs times the chunk with its four planes of warm-up (the shorter list of chunks on a tie).
   // With the 32 x 16 tiles of before and chunks of 64, then of the rule: 128^3 87 -> 50 us (32
   // planes), 192x64x128 83 -> 37 us (22), 256^3 345 -> 331 us (32); with the 32 x 24 tiles 45 us
   // (22), 36 us (16) and 254 us (52), 512^3 104 planes.
+  // The boxes of an ensemble share the chip: the rule takes the columns of all of them, as if they were
+  // boxes like this one.  A chunk of 64 whatever the number of boxes left SMs idle (steps, from 64
+  // to the rule's: 16 boxes of 64^3 432 -> 405 us, 4 of 64^3 224 -> 142, 2 of 128^3 423 -> 392).
   // Results do not depend on the chunk.
-  return best_zchunk(g.nz, cols, 148, 4);
+  return best_zchunk(g.nz, (long long)(cols * share), 148, 4);
 }
 
 dim3 phase_grid(const Geo& g, int zc) {
@@ -431,7 +428,7 @@ template <typename L> static cudaError_t launch_one(const PhaseArgs& a, cudaStre
   PhaseArgs b = a;
   b.dta = a.g.dt * a.alpha;
   b.dtb = a.g.dt * a.beta;
-  b.zchunk = phase_zchunk(a.g, a.zchunk, a.many);
+  b.zchunk = phase_zchunk(a.g, a.zchunk, a.share);
   const int zc = b.zchunk;
   if (zc % 2 || a.g.nz % 2) return cudaErrorInvalidValue;  // the plane loop runs two planes at a time
   kern<<<phase_grid(a.g, zc), L::PNT, smem, st>>>(b);

@@ -92,7 +92,7 @@ struct PhaseArgs {
   double alpha, beta;
   int clamp;            // 1: phi clamped to [0,1] before the log
   int zchunk;           // z planes per block (0: default)
-  bool many = false;    // the box shares the chip with others (default chunk)
+  double share = 1;     // cells of all boxes that share the chip, over this box's (default chunk)
   double dta = 0, dtb = 0;  // dt alpha, dt beta (set by launch_phase)
 };
 cudaError_t launch_phase(const PhaseArgs& a, cudaStream_t st);
@@ -107,7 +107,7 @@ template <typename A> struct BatchArgs {
   int* counter;
   double alpha, beta;
 };
-int phase_zchunk(const Geo& g, int requested, bool many);  // the z chunk launch_phase uses
+int phase_zchunk(const Geo& g, int requested, double share);  // the z chunk launch_phase uses
 dim3 phase_grid(const Geo& g, int zc);           // its tiles: x, y, z chunk
 enum class PhaseTiles { Tall, Flat, Wide };
 PhaseTiles phase_tiles(const Geo& g);            // ... of this shape; the boxes of one batched launch share it
@@ -124,14 +124,14 @@ struct MomArgs {
   const DevScalars* sc;
   double alpha, beta;
   int zchunk;                // z planes per block (0: default)
-  bool many = false;         // the box shares the chip with others (default chunk)
+  double share = 1;          // as in PhaseArgs
   // TMA tensor maps of u, v, w and phi^{n+1} (mom_field_maps); when `tma` is set the blocks whose
   // rings need no periodic wrap in x and y fill them with TMA boxes instead of per-thread copies
   int tma = 0;
   CUtensorMap tmu, tmv, tmw, tmphi;
 };
 cudaError_t launch_mom(const MomArgs& a, cudaStream_t st);
-int mom_zchunk(const Geo& g, int requested, bool many);  // the z chunk launch_mom uses
+int mom_zchunk(const Geo& g, int requested, double share);  // the z chunk launch_mom uses
 dim3 mom_grid(const Geo& g, int zc);           // its tiles: x, y, z chunk
 cudaError_t launch_mom_batch(const BatchArgs<MomArgs>& b, bool phi, int nsm, cudaStream_t st);
 // tensor map of an x-fastest nx*ny*nz float64 field with the ring box of the momentum kernels: u, v, w

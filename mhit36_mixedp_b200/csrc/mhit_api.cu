@@ -93,7 +93,7 @@ struct mhit_ctx {
   cudaGraphExec_t gexec[2] = {nullptr, nullptr};
   cudaEvent_t ev[2 * ST_COUNT] = {};
   int zchunk_phase = 0, zchunk_mom = 0;  // z planes per block of k_phase / k_mom (0: default)
-  bool in_ensemble = false;               // a box of an ensemble: its default z chunks are those of a shared chip
+  double share = 1.0;                     // cells of the box's ensemble, which share the chip, over its own
   long long label_bound = 0;              // test hook: union-find loop bound (0: the cell count)
   ZsolveTc* tcz = nullptr;                // tensor-core z solve (zsolve_tc = 1)
   CUtensorMap tm_u[2], tm_v[2], tm_w[2], tm_phi[2];  // k_mom's ring boxes over U, V, W, PHI[0..1]
@@ -258,7 +258,7 @@ static PhaseArgs phase_args(const mhit_ctx* c, double alpha, double beta, int cu
   a.beta = beta;
   a.clamp = c->prm.acdi_clamp;
   a.zchunk = c->zchunk_phase;
-  a.many = c->in_ensemble;
+  a.share = c->share;
   return a;
 }
 
@@ -281,7 +281,7 @@ static MomArgs mom_args(const mhit_ctx* c, double alpha, double beta, int cur) {
   a.alpha = alpha;
   a.beta = beta;
   a.zchunk = c->zchunk_mom;
-  a.many = c->in_ensemble;
+  a.share = c->share;
   a.tma = c->mom_tma;
   a.tmu = c->tm_u[cur];
   a.tmv = c->tm_v[cur];
@@ -1750,10 +1750,10 @@ static int ens_prepare_batch(mhit_ensemble* e) {
     mhit_ctx* c = e->box[b];
     for (int par = 0; par < 2; ++par) {
       PhaseArgs p = phase_args(c, 1.0, 0.0, par);
-      p.zchunk = phase_zchunk(c->g, c->zchunk_phase, true);
+      p.zchunk = phase_zchunk(c->g, c->zchunk_phase, c->share);
       pa[par].push_back(p);
       MomArgs m = mom_args(c, 1.0, 0.0, par);
-      m.zchunk = mom_zchunk(c->g, c->zchunk_mom, true);
+      m.zchunk = mom_zchunk(c->g, c->zchunk_mom, c->share);
       m.tma = 0;  // the tensor maps would be read from device memory: per-thread ring copies
       ma[par].push_back(m);
     }
@@ -1966,11 +1966,11 @@ int mhit_ensemble_create(const mhit_params* params, int nbox, mhit_ensemble** ou
   for (int b = 0; b < nbox && rc == MHIT_OK; ++b) {
     mhit_ctx* c = nullptr;
     rc = mhit_init(&params[b], &c);
-    if (rc == MHIT_OK) {
-      c->in_ensemble = true;
-      e->box.push_back(c);
-    }
+    if (rc == MHIT_OK) e->box.push_back(c);
   }
+  size_t cells = 0;
+  for (const mhit_ctx* c : e->box) cells += c->n;
+  for (mhit_ctx* c : e->box) c->share = (double)cells / c->n;
   if (rc == MHIT_OK) {
     cudaError_t err = cudaStreamCreateWithFlags(&e->st, cudaStreamNonBlocking);
     if (err == cudaSuccess) err = cudaEventCreateWithFlags(&e->fork, cudaEventDisableTiming);
