@@ -2092,6 +2092,8 @@ int mhit_ensemble_autotune(mhit_ensemble* e, int trials, int* nlanes_out) {
     }
     if ((rc = reset_state(c))) return rc;
   }
+  // the per-box lanes first: a new ensemble is set to the batched schedule
+  e->batched = false;
   int best_l = e->nbox;
   double best_t = 1e30;
   for (int nl = 1;; nl *= 2) {
