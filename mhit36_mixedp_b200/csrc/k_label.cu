@@ -16,10 +16,15 @@
 // that the host turns into an error status instead of looping.
 //
 // Most cells are background, so every pass is a scan of the label field (0.08 ms at 512^3, 4 bytes
-// per cell): the threads take four consecutive cells (nx is a multiple of 16) with one 16-byte load
-// and skip the groups without a masked cell.  One cell per thread and iteration was bound by the
-// latency of those loads: merge 0.51, flatten and count 0.32, number 0.38, statistics 1.03 ms for
-// 256 drops at 512^3.
+// per cell), and with one cell per thread and iteration the latency of those loads bounds it.  The
+// mask and the statistics take four consecutive cells per thread (nx is a multiple of 16) with one
+// 16-byte load and skip the groups without a masked cell; the merge and the flatten pass have four
+// loads of consecutive lanes in flight, because there the masked cells' work counts: with four
+// consecutive cells per thread, one after the other, they took up to four times as long.  Merge and
+// flatten, us, one cell per thread / four consecutive / now (64 drops at 64^3 and 256^3, all of
+// 64^3, a 256^3 box filled to a third, 64 drops at 512^3):
+//   18 / 58 / 19    157 / 224 / 138    97 / 473 / 107    503 / 1193 / 611    837 / 706 / 601
+// and the statistics 14 / 8, 184 / 82, 92 / 25, 1790 / 460, 1099 / 417 (the first and the last two).
 #include "common.cuh"
 #include "kernels.h"
 
@@ -33,6 +38,8 @@ __constant__ int8_t c_fwd[13][3] = {{0, 0, 1},  {0, 1, 0},  {1, 0, 0},  {0, 1, 1
 // Root of x with path halving: each visited node is re-pointed at its grandparent.  A node's
 // ancestors stay its ancestors (roots are only ever hung under smaller roots) and parents only
 // decrease, so a plain store of the grandparent is safe under concurrent links and halvings.
+// ATOMIC: stored by an atomicMin (k_lab_flatten).
+template <bool ATOMIC = false>
 __device__ __forceinline__ int find_root(int* lab, int x, long long bound, int* err) {
   volatile int* vl = lab;  // parents change under concurrent links: read them from L2
   for (long long it = 0; it < bound; ++it) {
@@ -40,7 +47,8 @@ __device__ __forceinline__ int find_root(int* lab, int x, long long bound, int* 
     if (y == x) return x;
     const int z = vl[y];
     if (z == y) return y;
-    vl[x] = z;
+    if (ATOMIC) atomicMin(&lab[x], z);
+    else vl[x] = z;
     x = z;
   }
   atomicExch(err, 1);
@@ -64,19 +72,6 @@ __device__ __forceinline__ void unite(int* lab, int a, int b, long long bound, i
   atomicExch(err, 1);
 }
 
-// Root of x without re-pointing anything (the flatten pass: a concurrent halving could put back a
-// grandparent over a root that another thread has just stored).
-__device__ __forceinline__ int walk_root(const int* lab, int x, long long bound, int* err) {
-  const volatile int* vl = lab;
-  for (long long it = 0; it < bound; ++it) {
-    const int y = vl[x];
-    if (y == x) return x;
-    x = y;
-  }
-  atomicExch(err, 1);
-  return x;
-}
-
 __global__ void k_lab_init(const double* __restrict__ phi, double thresh, int* __restrict__ lab, int n) {
   for (int c = 4 * (blockIdx.x * blockDim.x + threadIdx.x); c < n; c += 4 * gridDim.x * blockDim.x) {
     const double2 p = *reinterpret_cast<const double2*>(phi + c), q = *reinterpret_cast<const double2*>(phi + c + 2);
@@ -86,16 +81,23 @@ __global__ void k_lab_init(const double* __restrict__ phi, double thresh, int* _
   }
 }
 
+// R: cells per lane and iteration, each a row of 32 cells of the warp.  Four from 2^22 cells on (512^3
+// 605 -> 494 us, 256^3 122 -> 106 for 64 drops); below, where that leaves too few warps, one (128^3 87 ->
+// 71, 64^3 28 -> 14).
+template <int R>
 __global__ void k_lab_merge(int* lab, int nx, int ny, int nz, int nfwd, long long bound, int* err) {
   const int n = nx * ny * nz;
-  for (int c4 = 4 * (blockIdx.x * blockDim.x + threadIdx.x); c4 < n; c4 += 4 * gridDim.x * blockDim.x) {
-    // parents change under concurrent links, masked (>= 0) or not does not
-    const int4 l = __ldcg(reinterpret_cast<const int4*>(lab + c4));
-    if ((l.x & l.y & l.z & l.w) < 0) continue;  // all four negative
-    const int i0 = c4 % nx, j = (c4 / nx) % ny, k = c4 / (nx * ny);
-    for (int e = 0; e < 4; ++e) {
-      if ((e == 0 ? l.x : (e == 1 ? l.y : (e == 2 ? l.z : l.w))) < 0) continue;
-      const int c = c4 + e, i = i0 + e;
+  const int lane = threadIdx.x & 31, warps = gridDim.x * (blockDim.x >> 5);
+  for (int c0 = 32 * R * (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) + lane; c0 < n; c0 += 32 * R * warps) {
+    int l[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) l[r] = __ldcg(lab + c0 + 32 * r);  // n is a multiple of 128
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      // parents change under concurrent links, masked (>= 0) or not does not
+      if (l[r] < 0) continue;
+      const int c = c0 + 32 * r;
+      const int i = c % nx, j = (c / nx) % ny, k = c / (nx * ny);
       for (int q = 0; q < nfwd; ++q) {
         int ii = i + c_fwd[q][2], jj = j + c_fwd[q][1], kk = k + c_fwd[q][0];
         ii = ii < 0 ? ii + nx : (ii >= nx ? ii - nx : ii);
@@ -110,28 +112,33 @@ __global__ void k_lab_merge(int* lab, int nx, int ny, int nz, int nfwd, long lon
 
 constexpr int LTHREADS = 256, LCHUNK = 8192;  // threads and cells of a block of the chunked passes
 
-// Every masked cell points at its root afterwards; counts the roots of each chunk of LCHUNK
-// consecutive cells (one block per chunk).
-__global__ void __launch_bounds__(LTHREADS) k_lab_flatten(int* lab, int n, long long bound, int* err,
+// Every masked cell points at its root afterwards; adds the roots of each chunk of LCHUNK consecutive
+// cells to its count (zero before).  A block takes `part` cells, a divisor of LCHUNK.  Halvings store
+// with an atomicMin: a plain store could put back a grandparent over a root that the cell's own
+// thread has just stored.  Without halving, a chain is walked by every cell on it (rods of 64 cells
+// at 64^3 50 us, now 14).
+__global__ void __launch_bounds__(LTHREADS) k_lab_flatten(int* lab, int n, int part, long long bound, int* err,
                                                           int* __restrict__ counts) {
   __shared__ int s;
   if (threadIdx.x == 0) s = 0;
   __syncthreads();
-  const int c0 = blockIdx.x * LCHUNK, c1 = min(c0 + LCHUNK, n);
+  const int p0 = blockIdx.x * part, p1 = min(p0 + part, n);
   int local = 0;
-  for (int c = c0 + 4 * threadIdx.x; c < c1; c += 4 * LTHREADS) {
-    const int4 l = __ldcg(reinterpret_cast<const int4*>(lab + c));
-    const int v[4] = {l.x, l.y, l.z, l.w};
+  for (int c = p0 + threadIdx.x; c < p1; c += 4 * LTHREADS) {
+    int l[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      if (v[e] < 0) continue;
-      if (v[e] == c + e) ++local;  // roots stay roots in this pass
-      else lab[c + e] = walk_root(lab, v[e], bound, err);
+    for (int r = 0; r < 4; ++r) l[r] = c + r * LTHREADS < p1 ? __ldcg(lab + c + r * LTHREADS) : -1;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      if (l[r] < 0) continue;
+      const int e = c + r * LTHREADS;
+      if (l[r] == e) ++local;  // roots stay roots in this pass
+      else lab[e] = find_root<true>(lab, l[r], bound, err);
     }
   }
   if (local) atomicAdd(&s, local);
   __syncthreads();
-  if (threadIdx.x == 0) counts[blockIdx.x] = s;
+  if (threadIdx.x == 0 && s) atomicAdd(&counts[p0 / LCHUNK], s);
 }
 
 // Number the roots in index order (offsets: the first number of each chunk and the total; chunks
@@ -283,8 +290,11 @@ cudaError_t launch_label_components(const LabelArgs& a, cudaStream_t st) {
   // the loops' bound: the cell count (no chain or retry sequence is longer), or a smaller test
   // bound that makes a legitimate chain run out and exercises the error path
   const long long bound = a.bound > 0 ? a.bound : n;
-  k_lab_merge<<<grid, 256, 0, st>>>(a.lab, a.nx, a.ny, a.nz, a.connectivity == 26 ? 13 : 3, bound, a.err);
-  k_lab_flatten<<<label_chunks(n), LTHREADS, 0, st>>>(a.lab, n, bound, a.err, a.counts);
+  const auto merge = n >= (1 << 22) ? k_lab_merge<4> : k_lab_merge<1>;
+  merge<<<grid, 256, 0, st>>>(a.lab, a.nx, a.ny, a.nz, a.connectivity == 26 ? 13 : 3, bound, a.err);
+  // whole chunks where they fill the chip (eight blocks per SM); 64^3 has 32 of them
+  const int part = label_chunks(n) >= 148 * 8 ? LCHUNK : LCHUNK / 8;
+  k_lab_flatten<<<(n + part - 1) / part, LTHREADS, 0, st>>>(a.lab, n, part, bound, a.err, a.counts);
   return cudaGetLastError();
 }
 

@@ -212,7 +212,7 @@ struct LabelArgs {
   double thresh;
   int connectivity;             // 6 or 26
   int* lab;                     // n ints of scratch: parents, then the drop encoding
-  int* counts;                  // roots per chunk of cells, then the chunks' first drop numbers
+  int* counts;                  // roots per chunk of cells (zero before), then the chunks' first drop numbers
   int* err;                     // set when a bounded union-find loop ran out
   const double *u, *v, *w;      // stored velocity (lazy mean in sc)
   const DevScalars* sc;

@@ -1279,7 +1279,7 @@ int mhit_label_drops(mhit_ctx* c, double thresh, int connectivity, mhit_drop* dr
     }
   }
   MHIT_CUDA_TRY(cudaMemcpyAsync(trig, th.data(), sizeof(double) * trig_n, cudaMemcpyHostToDevice, c->st));
-  MHIT_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(int), c->st));
+  MHIT_CUDA_TRY(cudaMemsetAsync(counts, 0, sizeof(int) * (nch + 1), c->st));  // and err
   LabelArgs a;
   a.nx = nx;
   a.ny = ny;

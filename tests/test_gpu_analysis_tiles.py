@@ -1,7 +1,7 @@
 """The field analysis where its grouping of cells can go wrong.
 
-Labelling takes four consecutive cells per thread and 128 per warp: random masks put several drops
-into one group of four and dozens into one warp.  The diagnostics march 32 x 16 tiles and the spectrum
+Labelling takes four consecutive cells per thread or four rows of 32 per warp (the larger boxes' merge):
+random masks put several drops into one group of four and dozens into one warp.  The diagnostics march 32 x 16 tiles and the spectrum
 sums runs of equal shells in a warp: boxes that leave partial tiles, rows shorter than a warp and
 more shells than eight warps' histograms hold.  Sums of N terms in FP64 against numpy's: 1e-12.
 """
@@ -17,7 +17,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("conn", [6, 26])
-@pytest.mark.parametrize("shape,fill", [((16, 16, 16), 0.1), ((64, 16, 32), 0.3), ((192, 16, 16), 0.05)])
+@pytest.mark.parametrize("shape,fill", [((16, 16, 16), 0.1), ((64, 16, 32), 0.3), ((192, 16, 16), 0.05),
+                                        ((256, 64, 256), 0.3)])
 def test_labels_of_random_masks(gpu, shape, fill, conn):
     nx, ny, nz = shape
     rng = np.random.default_rng(11)
