@@ -1518,8 +1518,11 @@ int mhit_energy_spectrum(mhit_ctx* c, double* E, int nbins) {
     ty = c->tw64[1];
     tz = c->tw64[2];
   }
-  // the shell sums, then every block's histogram
-  if ((rc = grow_buffer(&c->spec_acc, &c->spec_acc_bytes, ((size_t)spectrum_blocks(g) + 1) * nbins * sizeof(double))))
+  // the shell sums, then every block's histogram; the shells past the corner of the wavenumber box,
+  // (nx/2, nx/2, nx/2) in the units of the x axis, stay zero without a histogram
+  const int nsh = std::min(nbins, (int)ceil(sqrt(3.0) * g.nx / 2) + 2);
+  if ((rc = grow_buffer(&c->spec_acc, &c->spec_acc_bytes,
+                        (nbins + (size_t)spectrum_blocks(g) * nsh) * sizeof(double))))
     return rc;
   double* dE = static_cast<double*>(c->spec_acc);
   MHIT_CUDA_TRY(cudaMemsetAsync(dE, 0, (size_t)nbins * sizeof(double), c->st));
@@ -1542,7 +1545,7 @@ int mhit_energy_spectrum(mhit_ctx* c, double* E, int nbins) {
     MHIT_CUDA_TRY(poisson_stage(a, PSTAGE_XFWD, c->st));
     MHIT_CUDA_TRY(poisson_stage(a, PSTAGE_YFWD, c->st));
     MHIT_CUDA_TRY(poisson_stage(a, PSTAGE_ZFWD, c->st));
-    MHIT_CUDA_TRY(launch_spectrum_bin(static_cast<const Cx<double>*>(spec), g, c->sc, comp, nbins,
+    MHIT_CUDA_TRY(launch_spectrum_bin(static_cast<const Cx<double>*>(spec), g, c->sc, comp, nsh,
                                       dE + nbins, dE, c->st));
   }
   MHIT_CUDA_TRY(cudaMemcpyAsync(E, dE, (size_t)nbins * sizeof(double), cudaMemcpyDeviceToHost, c->st));
