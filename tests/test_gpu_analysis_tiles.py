@@ -18,7 +18,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("conn", [6, 26])
 @pytest.mark.parametrize("shape,fill", [((16, 16, 16), 0.1), ((64, 16, 32), 0.3), ((192, 16, 16), 0.05),
-                                        ((256, 64, 256), 0.3)])
+                                        ((256, 64, 256), 0.05)])
 def test_labels_of_random_masks(gpu, shape, fill, conn):
     nx, ny, nz = shape
     rng = np.random.default_rng(11)
@@ -29,9 +29,7 @@ def test_labels_of_random_masks(gpu, shape, fill, conn):
         got = s.label_drops(0.5, conn, labels=True)
     lab = orc.label_components(phi, 0.5, conn)
     ref = orc.drop_statistics(lab, u, v, w)
-    expect = np.zeros(phi.shape, dtype=np.int32)
-    for d, root in enumerate(ref["label"]):
-        expect[lab == root] = d + 1
+    expect = np.where(lab >= 0, np.searchsorted(ref["label"], lab) + 1, 0)  # roots in index order
     np.testing.assert_array_equal(got["labels"], expect)
     np.testing.assert_array_equal(got["cells"], ref["cells"])
     for key in ("u", "v", "w"):
