@@ -311,8 +311,6 @@ template <typename S, bool REV> __host__ __device__ constexpr int spbefore(int s
   for (int i = 0; i < s; ++i) p *= srad<S, REV>(i);
   return p;
 }
-template <int N, bool REV> __host__ __device__ constexpr int rad(int s) { return srad<Radix<N>, REV>(s); }
-template <int N, bool REV> __host__ __device__ constexpr int pbefore(int s) { return spbefore<Radix<N>, REV>(s); }
 template <int N, int B, int NT, int R> struct StageShape {
   static constexpr int NB = N / R * B;
   static constexpr int BPT = (NB + NT - 1) / NT;

@@ -88,22 +88,18 @@ template <typename T, int M, bool INC> __host__ __device__ constexpr size_t xc_s
 template <typename T, int M, bool INC> __host__ __device__ constexpr size_t xc_smem() {
   return xc_nb<T, M, INC>() * xc_buffer_bytes<T, M, INC>();
 }
-// where the loads go through registers: x pairs a stream thread loads before computing any of them
-template <typename T, int M, bool INC> __host__ __device__ constexpr int xc_pb() {
-  return xc_ng<T, M, INC>() == 2 ? 7 : 2;
-}
-// Where it fits as well (nx = 512), each stream thread stages its u, v, w pairs of the NEXT plane
-// in shared memory with cp.async, pair by pair as it finishes the current plane's pair (one
-// commit group per pair), so a whole plane's loads (~86 KB per SM) are in flight while the
-// current plane is projected and no registers hold them.
+// where the loads go through registers (one group): x pairs a stream thread loads before computing
+// any of them
+constexpr int XPB = 2;
+// With two groups each stream thread stages its u, v, w pairs of the NEXT plane in shared memory with
+// cp.async, pair by pair as it finishes the current plane's pair (one commit group per pair), so a
+// whole plane's loads (86 KB per SM at nx = 512) are in flight while the current plane is projected
+// and no registers hold them.
 template <typename T, int M, bool INC> __host__ __device__ constexpr size_t xc_uvw_bytes() {
   return (size_t)3 * xc_ns<M>() * xc_ppt<M>() * 16;
 }
-template <typename T, int M, bool INC> __host__ __device__ constexpr bool xc_uvw_shared() {
-  return xc_ng<T, M, INC>() == 2 && xc_smem<T, M, INC>() + xc_uvw_bytes<T, M, INC>() <= 227 * 1024;
-}
 template <typename T, int M, bool INC> __host__ __device__ constexpr size_t xc_smem_all() {
-  return xc_smem<T, M, INC>() + (xc_uvw_shared<T, M, INC>() ? xc_uvw_bytes<T, M, INC>() : 0);
+  return xc_smem<T, M, INC>() + (xc_ng<T, M, INC>() == 2 ? xc_uvw_bytes<T, M, INC>() : 0);
 }
 
 __device__ __forceinline__ void bar_sync(int id, int count) {
@@ -122,8 +118,6 @@ __global__ void __launch_bounds__(xc_nt<T, M, INC>(), 1) k_xinv_correct(const Xc
   constexpr int TL = (M + 1) * XL;         // elements of one tile buffer
   constexpr int NP = XO * M;               // x pairs projected per plane
   constexpr int PPT = xc_ppt<M>();         // ... per stream thread
-  constexpr int XPB = xc_pb<T, M, INC>();
-  constexpr bool UVS = xc_uvw_shared<T, M, INC>();
   constexpr int nx = 2 * M;
   constexpr int QL = XL * nx;              // floats of one predictor tile
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -220,7 +214,7 @@ __global__ void __launch_bounds__(xc_nt<T, M, INC>(), 1) k_xinv_correct(const Xc
     // pair m of plane index ip into its slots, as one commit group (empty for pairs without a cell,
     // and past the last plane, so every thread commits PPT groups per plane)
     auto stage_pair = [&](int ip, int m) {
-      if constexpr (UVS) {
+      if constexpr (NG == 2) {
         const int e = st + m * NS;
         if (ip < nplanes && (NP % NS == 0 || e < NP)) {
           const int l = e / M, n = e - l * M;
@@ -241,24 +235,20 @@ __global__ void __launch_bounds__(xc_nt<T, M, INC>(), 1) k_xinv_correct(const Xc
       // the plane below's buffer (NG == 2; not read for i = 0)
       const Cx<T>* sb = tiles + ((i + XNB - 1) % XNB) * TL;
       const float* qb = qtiles + ((i + XNB - 1) % XNB) * QL;
-      // pressure of pair m (tile position n, line l + 1) at the plane below
-      auto below = [&](int m, int n, int l) -> double2 {
-        if constexpr (NG == 2) {
-          const Cx<T> z = sb[sw<XL>(n, l + 1)];
-          if constexpr (INC) {
-            const float2 q = *reinterpret_cast<const float2*>(qb + (l + 1) * nx + 2 * n);
-            return make_double2((double)q.x + (double)z.x, (double)q.y + (double)z.y);
-          } else {
-            return make_double2((double)z.x, (double)z.y);
-          }
+      // pressure of the pair at tile position n, line l + 1, at the plane below
+      auto below = [&](int n, int l) -> double2 {
+        const Cx<T> z = sb[sw<XL>(n, l + 1)];
+        if constexpr (INC) {
+          const float2 q = *reinterpret_cast<const float2*>(qb + (l + 1) * nx + 2 * n);
+          return make_double2((double)q.x + (double)z.x, (double)q.y + (double)z.y);
         } else {
-          return pzr[m];
+          return make_double2((double)z.x, (double)z.y);
         }
       };
       const int k = k0 - 1 + i;
       const int kk = k < 0 ? k + nz : k;
       bar_sync(READY + i % XNB, PAIR);  // plane i's pressure (and predictor rows) are ready
-      if constexpr (UVS) {
+      if constexpr (NG == 2) {
 #pragma unroll
         for (int m = 0; m < PPT; ++m) {
           const int e = st + m * NS;
@@ -296,7 +286,7 @@ __global__ void __launch_bounds__(xc_nt<T, M, INC>(), 1) k_xinv_correct(const Xc
               // multi/main.f90:953-955, the expressions of k_correct
               const double u0 = uo.x - cc * (p0 - pxm) * dxi, u1 = uo.y - cc * (p1 - p0) * dxi;
               const double v0 = vo.x - cc * (p0 - py0) * dxi, v1 = vo.y - cc * (p1 - py1) * dxi;
-              const double2 pk = below(m, n, l);
+              const double2 pk = below(n, l);
               const double w0 = wo.x - cc * (p0 - pk.x) * dxi, w1 = wo.y - cc * (p1 - pk.y) * dxi;
               *reinterpret_cast<double2*>(U + o) = make_double2(u0, u1);
               *reinterpret_cast<double2*>(V + o) = make_double2(v0, v1);
@@ -309,7 +299,6 @@ __global__ void __launch_bounds__(xc_nt<T, M, INC>(), 1) k_xinv_correct(const Xc
               mv = fmax(mv, fmax(v0, v1));
               mw = fmax(mw, fmax(w0, w1));
             }
-            if constexpr (NG == 1) pzr[m] = make_double2(p0, p1);
           }
           // the slots are free (their values consumed above): the next plane's pair goes in
           stage_pair(i + 1, m);
@@ -369,7 +358,7 @@ __global__ void __launch_bounds__(xc_nt<T, M, INC>(), 1) k_xinv_correct(const Xc
                 // multi/main.f90:953-955, the expressions of k_correct
                 const double u0 = uo[mb].x - cc * (p0 - pxm) * dxi, u1 = uo[mb].y - cc * (p1 - p0) * dxi;
                 const double v0 = vo[mb].x - cc * (p0 - py0) * dxi, v1 = vo[mb].y - cc * (p1 - py1) * dxi;
-                const double2 pk = below(m, n, l);
+                const double2 pk = pzr[m];
                 const double w0 = wo[mb].x - cc * (p0 - pk.x) * dxi, w1 = wo[mb].y - cc * (p1 - pk.y) * dxi;
                 *reinterpret_cast<double2*>(U + o) = make_double2(u0, u1);
                 *reinterpret_cast<double2*>(V + o) = make_double2(v0, v1);
@@ -382,7 +371,7 @@ __global__ void __launch_bounds__(xc_nt<T, M, INC>(), 1) k_xinv_correct(const Xc
                 mv = fmax(mv, fmax(v0, v1));
                 mw = fmax(mw, fmax(w0, w1));
               }
-              if constexpr (NG == 1) pzr[m] = make_double2(p0, p1);
+              pzr[m] = make_double2(p0, p1);
             }
           }
         }
@@ -397,7 +386,7 @@ __global__ void __launch_bounds__(xc_nt<T, M, INC>(), 1) k_xinv_correct(const Xc
         }
       }
     }
-    if constexpr (UVS) __pipeline_wait_prior(0);  // no copy into the block's shared memory outlives it
+    if constexpr (NG == 2) __pipeline_wait_prior(0);  // no copy into the block's shared memory outlives it
   }
   // block reduction (fixed tree, as k_correct; the transform warps add the identities)
   __syncthreads();

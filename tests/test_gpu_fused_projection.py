@@ -5,9 +5,8 @@ By default a step transforms the y-inverted spectrum back along x inside the pro
 the step; it is transformed into its array, with the same arithmetic, only when something reads
 it.  The test hook ``mhit_debug_set_fused_projection(ctx, 0)`` runs the two passes apart.
 
-* Both must give the same fields up to rounding: the fused pass transforms in a radix-8
-  schedule (the separate pass in radix 16 at nx = 256 and 512), its butterflies may contract
-  multiply-adds differently, and it sums the per-block means over other blocks.  Bars, relative to
+* Both must give the same fields up to rounding: the projection's expressions may contract
+  multiply-adds differently, and the fused pass sums the per-block means over other blocks.  Bars, relative to
   each field's max: FP64 1e-13.  In the FP32 modes the two differ by FP32 rounding of the
   pressure (~6e-8 of it), which moves u by dt/rho dp/dx every step: the bars are those the FP32
   modes meet elsewhere (1e-7 for the fields against the FP64 step, 1e-4 for the FP32 pressure
@@ -15,8 +14,8 @@ it.  The test hook ``mhit_debug_set_fused_projection(ctx, 0)`` runs the two pass
   projected divergence must be as small either way.
   For every Poisson mode that fuses (FP64, FP32, incremental FP32), on cubic and non-cubic boxes
   whose ny is not a multiple of the fused pass's 7 lines per block (tail blocks), at nx = 192 (the
-  radix-3 schedule) and nx = 1024 (the pressure carried in registers instead of shared memory),
-  and at 256^3, the production tile shapes.
+  radix-3 schedule) and nx = 1024 (one transform group, the pressure of the plane below carried in
+  registers), and at 256^3, the production tile shapes.
 * The pressure must be the one the projection used: a download after a step equals a download
   after a call that reuses the spectrum (droplet labelling, energy spectrum) and after a second
   download, bit for bit.
