@@ -85,6 +85,7 @@ def test_pressure_survives_calls_that_reuse_the_spectrum(gpu, poisson):
     lap = "modified" if poisson == "fp32_incremental" else "exact"
     with Solver(Params(nx=n, dt=2e-4, mu=0.004, phiflag=1, radius=0.4, sigma=0.3, poisson=poisson,
                        laplacian=lap)) as s:
+        assert _lib.load().mhit_debug_set_fused_projection(s._ctx, 1) == 0
         s.upload(u, v, w, phi)
         s.step(3)
         s.label_drops()
@@ -99,6 +100,7 @@ def test_pressure_survives_calls_that_reuse_the_spectrum(gpu, poisson):
         got = s.download()
     with Solver(Params(nx=n, dt=2e-4, mu=0.004, phiflag=1, radius=0.4, sigma=0.3, poisson=poisson,
                        laplacian=lap)) as s:
+        assert _lib.load().mhit_debug_set_fused_projection(s._ctx, 1) == 0
         s.upload(u, v, w, phi)
         s.step(3)
         q1 = s.download(fields=("p",))["p"]

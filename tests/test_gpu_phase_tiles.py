@@ -2,7 +2,9 @@
 
 The stencils march tiles of x-y cells over chunks of z planes chosen from the grid size; these boxes
 leave a partial last tile in x or y, a short last chunk, or a chunk of two planes.  Each stage is one
-FP64 evaluation of the oracle's expressions, so the usual 1e-12 of the buffer's maximum applies.
+FP64 evaluation of the oracle's expressions, so the usual 1e-12 of the buffer's maximum applies.  The
+stages run twice: the first step is an Euler step with an empty history, the second (Adams-Bashforth)
+reads the right-hand sides of the first.
 """
 import numpy as np
 import pytest
@@ -34,14 +36,16 @@ def test_stencil_stages_on_ragged_boxes(gpu, shape, clamp):
     st = orc.new_state(op, u, v, w, phi=phi)
     with Solver(Params(**prm)) as s:
         s.upload(u, v, w, phi)
-        orc.phase_step(op, st)
-        s.run_stage("phase")
-        assert rel(s.buffer("phin"), st.phi) < TOL
-        assert rel(s.buffer("rphi"), st.rhsphi_o) < TOL
-        orc.momentum_step(op, st, orc.forcing_tables(op))
-        s.run_stage("momentum")
-        for f, name in (("un", "u"), ("vn", "v"), ("wn", "w")):
-            assert rel(s.buffer(f), getattr(st, name)) < TOL
+        for step in range(2):
+            orc.phase_step(op, st)
+            s.run_stage("phase")
+            assert rel(s.buffer("phin"), st.phi) < TOL, step
+            assert rel(s.buffer("rphi"), st.rhsphi_o) < TOL, step
+            orc.momentum_step(op, st, orc.forcing_tables(op))
+            s.run_stage("momentum")
+            for f, name in (("un", "u"), ("vn", "v"), ("wn", "w"), ("ru", "rhsu_o"), ("rv", "rhsv_o"), ("rw", "rhsw_o")):
+                assert rel(s.buffer(f), getattr(st, name)) < TOL, (step, f)
+            s.commit_step()
 
 
 @pytest.mark.parametrize("tma", [1, 0])
@@ -62,6 +66,34 @@ def test_momentum_of_a_large_box_without_the_phase_field(gpu, tma):
             assert rel(s.buffer(f), getattr(st, name)) < TOL
         for f, name in (("ru", "rhsu_o"), ("rv", "rhsv_o"), ("rw", "rhsw_o")):
             assert rel(s.buffer(f), getattr(st, name)) < TOL
+
+
+@pytest.mark.parametrize("tma", [1, 0])
+def test_momentum_of_a_large_box_over_two_chunks(gpu, tma):
+    """The large boxes' kernel over two z chunks and an Adams-Bashforth step: against the oracle, and
+    bit for bit against the general kernel.  Without forcing, and periodic in half the box's y length,
+    the box holds two copies of a box of half its cells, which takes the general kernel."""
+    nx, ny, nz = 512, 512, 128
+    u, v, w = synth.solenoidal_velocity(nx, 3, ny=ny // 2, nz=nz)
+    prm = dict(nx=nx, nz=nz, dt=1e-4, mu=0.004, f1=0.0, f2=0.0, f3=0.0)
+    op = orc.Params(ny=ny // 2, **prm)
+    st = orc.new_state(op, u, v, w)
+    twice = [np.concatenate([a, a], axis=1) for a in (u, v, w)]
+    with Solver(Params(ny=ny, **prm)) as s, Solver(Params(ny=ny // 2, **prm)) as half:
+        assert _lib.load().mhit_debug_set_mom_tma(s._ctx, tma) == 0
+        s.upload(*twice)
+        half.upload(u, v, w)
+        for step in range(2):
+            orc.momentum_step(op, st, orc.forcing_tables(op))
+            for one in (s, half):
+                one.run_stage("momentum")
+            for f, name in (("un", "u"), ("vn", "v"), ("wn", "w"), ("ru", "rhsu_o"), ("rv", "rhsv_o"), ("rw", "rhsw_o")):
+                h, got = half.buffer(f), s.buffer(f)
+                assert rel(h, getattr(st, name)) < TOL, (step, f)
+                np.testing.assert_array_equal(got[:, : ny // 2], h, err_msg=f)
+                np.testing.assert_array_equal(got[:, ny // 2 :], h, err_msg=f)
+            for one in (s, half):
+                one.commit_step()
 
 
 def test_phase_field_at_the_ends_of_the_logarithm(gpu):
