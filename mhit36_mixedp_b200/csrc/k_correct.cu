@@ -188,14 +188,12 @@ __global__ void __launch_bounds__(1024) k_finalize(const double* __restrict__ pa
 // z planes per block: 64 where that still leaves eight waves of two blocks on each of the 148
 // SMs (each chunk re-reads the p plane below it: 1.106 against 1.135 ms FP32, 1.209 against
 // 1.250 ms FP64 at 512^3), otherwise CZC, halved while the grid leaves SMs without a block (64^3:
-// 19 us with 16 planes, 15 us with 4), from 4 to 2 only while half of them are without: the plane read
-// below each chunk is then half of what a block does.  4 and 2 planes, us per step: 64^3 39.6 and 40.2,
-// 16 boxes of 64^3 370 and 377; 64x64x128, where 8 planes fill 128 SMs, 51.8 and with 4 planes 50.5.
+// 19 us with 16 planes, 15 us with 2)
 static int correct_chunk(const Geo& g) {
   const long long cols = (long long)((g.nx + CTX - 1) / CTX) * ((g.ny + CTY - 1) / CTY);
   if (cols * ((g.nz + 63) / 64) >= 8 * 148 * 2) return 64;
   int zc = CZC;
-  while (zc > 2 && cols * ((g.nz + zc - 1) / zc) < (zc > 4 ? 148 : 74)) zc /= 2;
+  while (zc > 2 && cols * ((g.nz + zc - 1) / zc) < 148) zc /= 2;
   return zc;
 }
 
