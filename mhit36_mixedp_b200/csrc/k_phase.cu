@@ -151,7 +151,8 @@ __device__ __forceinline__ void phase_tile(const PhaseArgs& a, double dta, doubl
   // how the compiler contracts each copy of the loop body.
   auto F_of = [&](double dx, double dy, double dz, double ph, double ps, double& fx, double& fy, double& fz) {
     const double n2 = __fma_rn(dz, dz, __fma_rn(dy, dy, __dmul_rn(dx, dx)));
-    const double normag = (n2 != 0.0 && n2 != INFINITY) ? rsqrt_fast(n2) : 0.0;  // NaN stays NaN
+    // clamped, psi is finite; else an infinite n2 gives 0 and NaN stays NaN
+    const double normag = (CLAMP ? n2 > 0.0 : n2 != 0.0 && n2 != INFINITY) ? rsqrt_fast(n2) : 0.0;
     const double val = clampv(ph);
     const double tt = (ps == ps) ? __fma_rn(2.0, val, -1.0) * TNORM : ps;
     const double fac = __dmul_rn(__dmul_rn(0.25, __fma_rn(-tt, tt, 1.0)), normag);
