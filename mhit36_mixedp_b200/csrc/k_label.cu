@@ -142,8 +142,8 @@ __global__ void __launch_bounds__(LTHREADS) k_lab_flatten(int* lab, int n, int p
 }
 
 // Number the roots in index order (offsets: the first number of each chunk and the total; chunks
-// without a root, nearly all of them, have nothing to do): the root of drop d (0-based) gets -(d + 2), so that any cell
-// finds its drop as -lab[lab[c]] - 2 (or -lab[c] - 2 at the root itself)
+// without a root, nearly all of them, have nothing to do): the root of drop d (0-based) gets
+// -(d + 2), so that any cell finds its drop as -lab[lab[c]] - 2 (or -lab[c] - 2 at the root itself)
 __global__ void k_lab_number(int* __restrict__ lab, int n, const int* __restrict__ offsets) {
   __shared__ int warp_tot[LTHREADS / 32];
   __shared__ int base;

@@ -105,9 +105,9 @@ __device__ __forceinline__ int pmod_int(int x, int n) {
 // last z force in registers instead of reading them from the rings again, 9 of 49 shared loads per
 // cell: the shared-memory pipe bounds the kernel (ncu: 79% of its wavefronts at 61% of the DRAM
 // bandwidth).  The same bits; 2.81 -> 2.75 ms at 512^3 and 386 -> 370 us at 256^3 on one box, 62 -> 58
-// us at 128^3.  Without the phase field nothing changes.  The batched kernel, whose arguments
-// take registers (they come from device memory), spills with it (ensemble of 32 boxes 4.55 -> 4.87
-// ms) and reads the rings.
+// us at 128^3.  Without the phase field, where u, v, w are carried too, the time does not change.  The
+// batched kernel, whose arguments take registers (they come from device memory), spills with it
+// (ensemble of 32 boxes 4.55 -> 4.87 ms) and reads the rings.
 template <bool PHI, bool CARRY>
 __device__ __forceinline__ void mom_tile(const MomArgs& a, double alpha, double beta, int bx, int by, int bz,
                                          unsigned char* smraw) {

@@ -106,7 +106,8 @@ struct mhit_ctx {
   //   256^3        849 / 789, 691 / 664, 785 / 721     256x256x64   234 / 215, 192 / 183, 217 / 202
   //   256x64x64     73 / 79,   69 / 74,   82 / 86      192^3        399 / 389, 326 / 314, 366 / 348
   //   192x64x128   100 / 101,  90 / 91,   98 / 99      128^3        123 / 122, 105 / 110, 115 / 117
-  //   64x512x512   858 / 947, 715 / 806, 788 / 908
+  //   64x512x512   858 / 947, 715 / 806, 788 / 908          256x16x1024   246 / 237, 208 / 207, 233 / 225
+  //   512x32x256   240 / 224, 201 / 190, 221 / 203          192x32x1024   353 / 339, 302 / 291, 342 / 326
   // (at 1024^3, where k_correct streams at 96% of the copy peak, the separate passes win).  The fused
   // pass leaves the pressure in the spectrum only: after such a step p_lazy is set, and whatever
   // reads the pressure or reuses the spectrum first materialises it (materialise_pressure).

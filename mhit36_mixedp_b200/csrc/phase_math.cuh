@@ -6,15 +6,15 @@
 
 namespace mhit {
 
-// log(a/b) for finite b > 0 and a > 0 (a = 0: -inf, a < 0 or NaN: NaN), to an ulp or two, without
-// branches, conversions or a separate quotient: with k the integer nearest to the difference of
+// log(a/b) for finite b > 0 and a > 0 (a = 0: -inf, a < 0 or NaN: NaN), to two ulps, without branches,
+// conversions or a separate quotient: with k the integer nearest to the difference of
 // the operands' piecewise-linear log2 (exponent and mantissa fields of the high words) and
 // a' = a 2^-k, a'/b lies in [0.66, 1.51] and
 //   log(a/b) = k log 2 + 2 atanh(s),  s = (a' - b)/(a' + b), |s| < 0.201,
 // a' - b exact (Sterbenz).  2 atanh(s) = 2 s (1 + z Q(z)), z = s^2, Q the degree-7 interpolant of
 // the series 1/3 + z/5 + z^2/7 + ... at the Chebyshev nodes of [0, 0.0415] (2^-60 of the sum).
 // The quotient is one Newton-Raphson step on the approximate reciprocal and one residual
-// correction.
+// correction (Markstein); log 2 is split in two so that its products with k are exact (Cody and Waite).
 template <bool POSITIVE> __device__ __forceinline__ double log_ratio(double a, double b) {
   const int ha = __double2hiint(a), hb = __double2hiint(b);
   const int k = (int)((unsigned)ha - (unsigned)hb + (1u << 19)) >> 20;
@@ -45,7 +45,8 @@ template <bool POSITIVE> __device__ __forceinline__ double log_ratio(double a, d
   return a > 0.0 ? l : (a == 0.0 ? -INFINITY : NAN);
 }
 
-// 1/sqrt(x) for normal x > 0: the approximate reciprocal square root and one third-order step
+// 1/sqrt(x) for normal x > 0 to 2^-52: the approximate reciprocal square root y and one Householder step
+// of third order, y (1 + e/2 + 3 e^2/8) with e = 1 - x y^2
 __device__ __forceinline__ double rsqrt_fast(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
